@@ -116,9 +116,12 @@ def _cpp_str(s: str) -> str:
 
 def _traits(tf) -> str:
     ns = tf.namespace
+    settled = "de_step<T, P>(c, pos, p, settled)" if tf.settles else "de_step<T, P>(c, pos, p)"
     return f"""struct F_{ns} {{
+  static constexpr bool kSettles = {'true' if tf.settles else 'false'};
   template <class T, class P> static ND_DEV_INLINE int32_t iterations(const P& p) {{ return {ns}::de_iterations<T, P>(p); }}
   template <class T, class P> static ND_DEV_INLINE ndw::IterCarry<T> step(ndw::IterCarry<T> c, ndw::v3<T> pos, const P& p) {{ return {ns}::de_step<T, P>(c, pos, p); }}
+  template <class T, class P> static ND_DEV_INLINE ndw::IterCarry<T> step(ndw::IterCarry<T> c, ndw::v3<T> pos, const P& p, bool& settled) {{ return {ns}::{settled}; }}
   template <class T, class P> static ND_DEV_INLINE T finalize(ndw::IterCarry<T> c) {{ return {ns}::de_finalize<T, P>(c); }}
 }};
 """

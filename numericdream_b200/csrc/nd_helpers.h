@@ -114,9 +114,13 @@ ND_HD_INLINE void sin_cos(double x, double& s, double& c) { ::sincos(x, &s, &c);
 
 // template.wgsl:1013 (BULB_BAILOUT) and 1019-1031: one Mandelbulb power step in
 // spherical coordinates (theta from +z, phi = atan2(y, x)); no-op once r > 2.
-template <class T> ND_HD_INLINE IterCarry<T> bulb_power_step(IterCarry<T> c, v3<T> add, T power) {
+// settled: set when the step returned its carry as it was.
+template <class T> ND_HD_INLINE IterCarry<T> bulb_power_step(IterCarry<T> c, v3<T> add, T power, bool& settled) {
   const T r = length(c.z);
-  if (r > T(2)) return c;
+  if (r > T(2)) {
+    settled = true;
+    return c;
+  }
   const T theta = acos(clamp(c.z.z / r, T(-1), T(1))) * power;
   const T phi = atan2(c.z.y, c.z.x) * power;
   const T rp = pow(r, power - T(1));
@@ -127,6 +131,10 @@ template <class T> ND_HD_INLINE IterCarry<T> bulb_power_step(IterCarry<T> c, v3<
   sin_cos(phi, sp, cp);
   const v3<T> z = v3<T>(st * cp, st * sp, ct) * zr + add;
   return IterCarry<T>{z, dr};
+}
+template <class T> ND_HD_INLINE IterCarry<T> bulb_power_step(IterCarry<T> c, v3<T> add, T power) {
+  bool settled;
+  return bulb_power_step<T>(c, add, power, settled);
 }
 
 // template.wgsl:1033-1055: abs then sort components so that x >= y >= z.

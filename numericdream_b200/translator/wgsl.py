@@ -723,6 +723,10 @@ TEMPLATE_FUNCS = {
     "smix": ([F32, F32, F32], F32),
 }
 
+# helpers that return the carry they were given once the orbit has escaped, with an
+# overload in nd_helpers.h that says so (`settled`)
+SETTLING_FUNCS = {"bulb_power_step"}
+
 _FLOAT_UNARY = {"sin", "cos", "tan", "asin", "acos", "atan", "sinh", "cosh", "tanh", "exp", "exp2",
                 "log", "log2", "sqrt", "inverseSqrt", "floor", "ceil", "round", "fract", "trunc",
                 "radians", "degrees", "saturate"}
@@ -797,6 +801,9 @@ class FormulaCompiler:
         self.calls: dict[str, set] = {}
         self.cur_fn = ""
         self.inv_fn = False  # translating de_step: track what is the same in every iteration
+        self.settling = False  # translating de_step's `settled` form
+        self.settles = False   # de_step has a return of its own carry
+        self.carry_te = None   # de_step's carry parameter
         for f in fns:
             if f.name in self.fn_sigs:
                 raise TranslateError(f"function {f.name} defined twice", f.line)
@@ -1595,6 +1602,13 @@ class FormulaCompiler:
         if isinstance(s, Return):
             if s.e is None:
                 return [pad + "return;"]
+            if self.carry_te is not None and (self.is_carry(s.e) or self.is_settling_call(s.e)):
+                self.settles = True
+                if self.settling:
+                    if self.is_carry(s.e):
+                        return [pad + "settled = true;", pad + f"return {self.expr(s.e).code};"]
+                    code = self.expr(s.e).code
+                    return [pad + f"return {code[:-1]}, settled);"]
             te = self.expr(s.e)
             if self.cur_ret.kind == "params":
                 raise TranslateError("returning Params is not supported", s.line)
@@ -1712,22 +1726,44 @@ class FormulaCompiler:
         return (f"template <class T, class P> ND_HD_INLINE {cpp_type(rty)} "
                 f"{cpp_name(f.name)}({', '.join(params)})")
 
-    def fn_body(self, f: FnDecl) -> list[str]:
+    def is_carry(self, e: Expr) -> bool:
+        """In de_step: is e the carry parameter (not a variable that shadows it)?"""
+        if not isinstance(e, Ident):
+            return False
+        for sc in reversed(self.scopes):
+            if e.name in sc:
+                return sc[e.name] is self.carry_te
+        return False
+
+    def is_settling_call(self, e: Expr) -> bool:
+        """In de_step: is e a helper that hands back the carry it was given once the orbit
+        has escaped (the hand-written helpers with a `settled` form)?"""
+        return (isinstance(e, Call) and e.name in SETTLING_FUNCS and e.name not in self.fn_sigs and
+                self.helper_ns == "ndw" and len(e.args) > 0 and self.is_carry(e.args[0]))
+
+    def fn_body(self, f: FnDecl, settling: bool = False) -> list[str]:
         ptys, rty = self.fn_sigs[f.name]
         self.cur_ret = rty
         self.cur_fn = f.name
+        self.settling = settling
+        self.carry_te = None
         # de_step(carry, pos, p): pos and the parameters are the same in every iteration
         self.inv_fn = f.name == "de_step" and len(ptys) == 3
         self.push()
         for k, (pn, pt) in enumerate(ptys):
             if pt.kind == "a" and pt.n == 8 and pt.elem == F32 and pn == "p":
                 pt = PARAMS
-            self.declare(pn, TE(pt, cpp_name(pn), None, lvalue=False, inv=self.inv_fn and k > 0), f.line)
+            te = TE(pt, cpp_name(pn), None, lvalue=False, inv=self.inv_fn and k > 0)
+            self.declare(pn, te, f.line)
+            if self.inv_fn and k == 0:
+                self.carry_te = te
         body = []
         for s in f.body:
             body.extend(self.stmt(s, 1))
         self.pop()
         self.inv_fn = False
+        self.settling = False
+        self.carry_te = None
         return body
 
     def is_inv(self, e: Expr) -> bool:
@@ -1781,6 +1817,12 @@ class FormulaCompiler:
             lines.append(self.fn_signature(f) + " {")
             lines.extend(body)
             lines.append("}")
+            if self.settles and name == "de_step":
+                # the same step, telling when it returned its own carry: de_step is a pure
+                # function of its arguments, so every later step returns that carry too
+                lines.append(self.fn_signature(f)[:-1] + ", bool& settled) {")
+                lines.extend(self.fn_body(f, settling=True))
+                lines.append("}")
         lines.append(f"}}  // namespace {self.ns}")
         return "\n".join(lines)
 
@@ -1793,6 +1835,7 @@ class TranslatedFormula:
     params: list
     source_hash: int
     features: set
+    settles: bool = False  # de_step has the form with the `settled` flag
 
 
 def _sanitize(name: str) -> str:
@@ -1815,7 +1858,8 @@ def translate(source: str, name: str) -> TranslatedFormula:
     ns = "ndf_" + _sanitize(name)
     comp = FormulaCompiler(fns, consts, ns)
     cpp = comp.emit()
-    return TranslatedFormula(name, ns, cpp, parse_formula_params(source), source_hash(source), comp.features)
+    return TranslatedFormula(name, ns, cpp, parse_formula_params(source), source_hash(source), comp.features,
+                             comp.settles)
 
 
 def translate_module(source: str, namespace: str, helper_ns: str = "ndw", contract: bool = True) -> str:

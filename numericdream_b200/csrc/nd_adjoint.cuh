@@ -49,7 +49,27 @@ struct AdjointArgs {
   double* dshade;                // nullable: dI/dtheta per G-buffer slot [slot][nparam + 3]
   int32_t param_idx[kMaxAdjParams];
   int32_t nparam;
+  int32_t num_sms;
+  int32_t inline_thetas;  // 0: adjoint_surface leaves the thetas to the second kernel
+  int64_t first;  // the rays [first, last) of the launch are worked on at a time
+  int64_t last;
+  unsigned* counts;     // entries in hits and in lit
+  int32_t* hits;        // contributing rays, as indices from first
+  struct LitRay* lit;   // those whose derivatives are not zero
 };
+
+// A listed ray that reached its derivatives: what the first adjoint kernel found.
+struct LitRay {
+  int32_t ray, view;
+  double denom, D[3];
+};
+// Rays worked on at a time: it bounds the scratch (44 bytes a ray).
+constexpr int64_t kAdjointRays = int64_t(1) << 22;
+// Blocks of 128 threads per SM the adjoint kernels are compiled for: surface FP32 and
+// FP64, thetas FP32 and FP64.  Measured for the thetas: FP32 5 / 6 / 8 blocks 978 / 1024 /
+// 1003 us a backward of 4 views of 512 x 512; FP64 2 / 3 / 4 blocks 1021 / 856 / 879 us
+// a backward of 2 views of 256 x 256.
+constexpr int kSurfaceBlocks32 = 6, kSurfaceBlocks64 = 4, kThetaBlocks32 = 5, kThetaBlocks64 = 3;
 
 // Parameter accessor with one dual tangent: parameter `seed` gets tangent 1.
 template <class S> struct DualParams {
@@ -70,6 +90,26 @@ ND_DEV_INLINE S de_dir(const DevView& v, D3 p, D3 tan, int seed) {
   return de_dir_full<Set, S>(v, p, tan, seed).d;
 }
 
+// Parameter accessor with dual tangents: parameter seed[i] has 1 in tangent i.
+template <class S, int N> struct DualsParams {
+  const float* v;
+  const int* seed;
+  ND_DEV_INLINE ndw::Duals<S, N> operator[](int i) const {
+    return ndw::mkds<N>(S(v[i]), [&](int k) { return i == seed[k] ? S(1) : S(0); });
+  }
+};
+
+// The DE of view v at p and its N derivatives along (position tangent tan[i], parameter
+// seed[i]).
+template <class Set, class S, int N>
+ND_DEV_INLINE ndw::Duals<S, N> de_dirs(const DevView& v, D3 p, const D3* tan, const int* seed) {
+  typedef ndw::Duals<S, N> DS;
+  const ndw::v3<DS> q(ndw::mkds<N>(S(p.x), [&](int i) { return S(tan[i].x); }),
+                      ndw::mkds<N>(S(p.y), [&](int i) { return S(tan[i].y); }),
+                      ndw::mkds<N>(S(p.z), [&](int i) { return S(tan[i].z); }));
+  return Set::template de_with<DS, DualsParams<S, N>>(v.code, q, DualsParams<S, N>{v.params, seed}, v).d;
+}
+
 // Largest |DE(p) - eps(t)| / eps(t) at a hit that is a root of the level set.  FP64
 // bisection leaves ~1e-13.  An FP32 DE near the surface carries rounding of ~1e-3 of
 // eps (12 iterations amplify each ulp by about dr), so FP32 tells only jumps above
@@ -82,132 +122,315 @@ ND_DEV_INLINE D3 axpy(D3 a, double s, D3 b) { return D3{a.x + s * b.x, a.y + s *
 ND_DEV_INLINE double dot3(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 ND_DEV_INLINE D3 axis(int i, double s) { return D3{i == 0 ? s : 0.0, i == 1 ? s : 0.0, i == 2 ? s : 0.0}; }
 
-// dI/dtheta_k of one hit ray (k < nparam: params[param_idx[k]]; then yaw, pitch,
-// dist), written to dI[0 .. nparam + 3).  Returns false when the pixel contributes
-// nothing (a back-lit normal, a degenerate gradient, a hit on a jump of the DE).
-template <class Set, class S>
-ND_DEV_INLINE bool adjoint_pixel(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
-                                 int64_t local, double t, double* dI) {
-  const int K = nparam + kPoseParams;
-  double ux, uy;
-  ray_uv(v, local, &ux, &uy);
-  const D3 w = D3{v.fwd[0] + v.right[0] * ux + v.up[0] * uy, v.fwd[1] + v.right[1] * ux + v.up[1] * uy,
-                  v.fwd[2] + v.right[2] * ux + v.up[2] * uy};
-  const double wn = sqrt(dot3(w, w));
-  const D3 d = ray_dir(v, local);  // w / |w| exactly as the forward computed it
-  const D3 p = fmadd(D3{v.org[0], v.org[1], v.org[2]}, d, t);
-  // value and gradient of the DE at the hit
-  const ndw::Dual<S> gx = de_dir_full<Set, S>(v, p, axis(0, 1.0), -1);
-  const D3 g = D3{double(gx.d), double(de_dir<Set, S>(v, p, axis(1, 1.0), -1)),
-                  double(de_dir<Set, S>(v, p, axis(2, 1.0), -1))};
-  const double eps_t = double(v.eps_coef) * t + double(v.eps_floor);
-  if (eps_t > 0.0 && !(fabs(double(gx.v) - eps_t) <= RootTol<S>::value * eps_t)) return false;
-  const double denom = dot3(g, d) - double(v.eps_coef);
+// The ray of a listed hit: what both adjoint kernels start from.
+struct AdjointRay {
+  double ux, uy, wn, t, hc, h;
+  D3 d, p;
+};
+ND_DEV_INLINE AdjointRay adjoint_ray(const DevView& v, int64_t local, double t) {
+  AdjointRay r;
+  ray_uv(v, local, &r.ux, &r.uy);
+  const D3 w = D3{v.fwd[0] + v.right[0] * r.ux + v.up[0] * r.uy, v.fwd[1] + v.right[1] * r.ux + v.up[1] * r.uy,
+                  v.fwd[2] + v.right[2] * r.ux + v.up[2] * r.uy};
+  r.wn = sqrt(dot3(w, w));
+  r.d = ray_dir(v, local);  // w / |w| exactly as the forward computed it
+  r.p = fmadd(D3{v.org[0], v.org[1], v.org[2]}, r.d, t);
+  r.t = t;
   const bool central = v.normal_h_coef > 0.0f;
-  const double hc = central ? double(v.normal_h_coef) : double(v.eps_coef);
-  const double h = central ? hc * t : double(v.eps_coef) * t + double(v.eps_floor);
-  // the normal's central-difference vector D
-  double Dv[3];
-  for (int i = 0; i < 3; ++i)
-    Dv[i] = double(de_dir_full<Set, S>(v, axpy(p, h, axis(i, 1.0)), D3{0, 0, 0}, -1).v) -
-            double(de_dir_full<Set, S>(v, axpy(p, -h, axis(i, 1.0)), D3{0, 0, 0}, -1).v);
-  const D3 D = D3{Dv[0], Dv[1], Dv[2]};
+  r.hc = central ? double(v.normal_h_coef) : double(v.eps_coef);
+  r.h = central ? r.hc * t : double(v.eps_coef) * t + double(v.eps_floor);
+  return r;
+}
+
+// dp/dtheta_k with t held fixed (k < nparam: params[param_idx[k]]; then yaw, pitch, dist).
+ND_DEV_INLINE D3 adjoint_tangent(const PoseTangents& T, const AdjointRay& r, int k, int nparam) {
+  D3 dorg = D3{0, 0, 0}, dd = D3{0, 0, 0};
+  if (k >= nparam && k < nparam + kPoseParams) {
+    const int j = k - nparam;
+    dorg = D3{T.dorg[j][0], T.dorg[j][1], T.dorg[j][2]};
+    const D3 dw = D3{T.dfwd[j][0] + r.ux * T.dright[j][0] + r.uy * T.dup[j][0],
+                     T.dfwd[j][1] + r.ux * T.dright[j][1] + r.uy * T.dup[j][1],
+                     T.dfwd[j][2] + r.ux * T.dright[j][2] + r.uy * T.dup[j][2]};
+    const double dd_par = dot3(r.d, dw);
+    dd = D3{(dw.x - r.d.x * dd_par) / r.wn, (dw.y - r.d.y * dd_par) / r.wn, (dw.z - r.d.z * dd_par) / r.wn};
+  }
+  return axpy(dorg, r.t, dd);
+}
+
+// dI/dtheta_k of one ray for the C thetas from k0 on.
+template <class Set, class S, int C>
+ND_DEV_INLINE void adjoint_thetas(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
+                                  const AdjointRay& r, double denom, const D3& D, int k0, double* dI) {
   const double Dn = sqrt(dot3(D, D));
-  if (!(Dn > 0.0) || denom == 0.0) return false;
   const D3 n = D3{D.x / Dn, D.y / Dn, D.z / Dn};
   const D3 L = D3{v.light[0], v.light[1], v.light[2]};
-  if (!(dot3(n, L) > 0.0)) return false;
-  for (int k = 0; k < K; ++k) {
-    D3 dorg = D3{0, 0, 0}, dd = D3{0, 0, 0};
-    int seed = -1;
-    if (k < nparam) {
-      seed = param_idx[k];
-    } else {
-      const int j = k - nparam;
-      dorg = D3{T.dorg[j][0], T.dorg[j][1], T.dorg[j][2]};
-      const D3 dw = D3{T.dfwd[j][0] + ux * T.dright[j][0] + uy * T.dup[j][0],
-                       T.dfwd[j][1] + ux * T.dright[j][1] + uy * T.dup[j][1],
-                       T.dfwd[j][2] + ux * T.dright[j][2] + uy * T.dup[j][2]};
-      const double dd_par = dot3(d, dw);
-      dd = D3{(dw.x - d.x * dd_par) / wn, (dw.y - d.y * dd_par) / wn, (dw.z - d.z * dd_par) / wn};
-    }
-    const D3 ptan0 = axpy(dorg, t, dd);  // dp/dtheta with t held fixed
-    const double a_k = double(de_dir<Set, S>(v, p, ptan0, seed));
+  if constexpr (C == 1) {
+    const int seed = k0 < nparam ? param_idx[k0] : -1;
+    const D3 ptan0 = adjoint_tangent(T, r, k0, nparam);
+    const double a_k = double(de_dir<Set, S>(v, r.p, ptan0, seed));
     const double dt = -a_k / denom;
-    const D3 dp = axpy(ptan0, dt, d);
-    const double dh = hc * dt;
+    const D3 dp = axpy(ptan0, dt, r.d);
+    const double dh = r.hc * dt;
     double dD[3];
     for (int i = 0; i < 3; ++i) {
       const D3 tp = axpy(dp, dh, axis(i, 1.0));
       const D3 tm = axpy(dp, -dh, axis(i, 1.0));
-      dD[i] = double(de_dir<Set, S>(v, axpy(p, h, axis(i, 1.0)), tp, seed)) -
-              double(de_dir<Set, S>(v, axpy(p, -h, axis(i, 1.0)), tm, seed));
+      dD[i] = double(de_dir<Set, S>(v, axpy(r.p, r.h, axis(i, 1.0)), tp, seed)) -
+              double(de_dir<Set, S>(v, axpy(r.p, -r.h, axis(i, 1.0)), tm, seed));
     }
     const double nd = n.x * dD[0] + n.y * dD[1] + n.z * dD[2];
     const D3 dn = D3{(dD[0] - n.x * nd) / Dn, (dD[1] - n.y * nd) / Dn, (dD[2] - n.z * nd) / Dn};
-    dI[k] = (1.0 - kSimpleAmbient) * dot3(L, dn);
+    dI[0] = (1.0 - kSimpleAmbient) * dot3(L, dn);
+  } else {
+    int seed[C];
+    D3 tan[C];
+    double dt[C], sum[C];  // sum: n . dD, then L . dD
+    for (int c = 0; c < C; ++c) {
+      seed[c] = k0 + c < nparam ? param_idx[k0 + c] : -1;
+      tan[c] = adjoint_tangent(T, r, k0 + c, nparam);
+      dt[c] = 0.0;
+    }
+    double nd[C];
+    for (int c = 0; c < C; ++c) sum[c] = nd[c] = 0.0;
+    // one call site: the evaluation at the hit (tap -1), then the six taps
+#pragma unroll 1
+    for (int tap = -1; tap < 6; ++tap) {
+      const int i = tap < 0 ? 0 : tap >> 1;
+      const double s = tap < 0 ? 0.0 : (tap & 1 ? -1.0 : 1.0);
+      D3 at[C];
+      for (int c = 0; c < C; ++c) {
+        const D3 dp = axpy(tan[c], dt[c], r.d);
+        at[c] = axpy(dp, s * r.hc * dt[c], axis(i, 1.0));
+      }
+      const ndw::Duals<S, C> e = de_dirs<Set, S, C>(v, axpy(r.p, s * r.h, axis(i, 1.0)), at, seed);
+      const double ni = i == 0 ? n.x : i == 1 ? n.y : n.z, Li = i == 0 ? L.x : i == 1 ? L.y : L.z;
+      for (int c = 0; c < C; ++c) {
+        if (tap < 0) {
+          dt[c] = -double(e.d[c]) / denom;
+        } else {
+          nd[c] += s * ni * double(e.d[c]);
+          sum[c] += s * Li * double(e.d[c]);
+        }
+      }
+    }
+    // L . dn with dn = (dD - n (n . dD)) / |D|
+    for (int c = 0; c < C; ++c) dI[c] = (1.0 - kSimpleAmbient) * (sum[c] - dot3(L, n) * nd[c]) / Dn;
   }
+}
+
+// What the derivatives along every theta share: g . d - coef and the normal's
+// central-difference vector D.  False when the pixel contributes nothing (a back-lit
+// normal, a degenerate gradient, a hit on a jump of the DE).
+//
+// The FP32 form ends in the loop over the first `thetas` derivatives, which the kernels
+// run zero times (adjoint_thetas computes them for the lit rays): the compiler contracts
+// the gradient's products into FMAs by what surrounds them, and with the loop there the
+// derivatives keep the rounding they had when one lane computed all of them.
+template <class Set, class S>
+ND_DEV_INLINE bool adjoint_surface(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
+                                   int thetas, const AdjointRay& r, double* denom, double* Dv, double* dI) {
+  // value and gradient of the DE at the hit
+  D3 g;
+  double value;
+  if constexpr (sizeof(S) == 8) {
+    const D3 axes[3] = {axis(0, 1.0), axis(1, 1.0), axis(2, 1.0)};
+    const int none[3] = {-1, -1, -1};
+    const ndw::Duals<S, 3> e = de_dirs<Set, S, 3>(v, r.p, axes, none);
+    value = e.v;
+    g = D3{e.d[0], e.d[1], e.d[2]};
+  } else {
+    const ndw::Dual<S> gx = de_dir_full<Set, S>(v, r.p, axis(0, 1.0), -1);
+    g = D3{double(gx.d), double(de_dir<Set, S>(v, r.p, axis(1, 1.0), -1)),
+           double(de_dir<Set, S>(v, r.p, axis(2, 1.0), -1))};
+    value = double(gx.v);
+  }
+  const double eps_t = double(v.eps_coef) * r.t + double(v.eps_floor);
+  if (eps_t > 0.0 && !(fabs(value - eps_t) <= RootTol<S>::value * eps_t)) return false;
+  *denom = dot3(g, r.d) - double(v.eps_coef);
+  // the normal's central-difference vector D
+  for (int i = 0; i < 3; ++i)
+    Dv[i] = double(de_dir_full<Set, S>(v, axpy(r.p, r.h, axis(i, 1.0)), D3{0, 0, 0}, -1).v) -
+            double(de_dir_full<Set, S>(v, axpy(r.p, -r.h, axis(i, 1.0)), D3{0, 0, 0}, -1).v);
+  const D3 D = D3{Dv[0], Dv[1], Dv[2]};
+  const double Dn = sqrt(dot3(D, D));
+  if (!(Dn > 0.0) || *denom == 0.0) return false;
+  const D3 n = D3{D.x / Dn, D.y / Dn, D.z / Dn};
+  if (!(dot3(n, D3{v.light[0], v.light[1], v.light[2]}) > 0.0)) return false;
+  if constexpr (sizeof(S) == 4)
+    for (int k = 0; k < thetas; ++k) adjoint_thetas<Set, S, 1>(v, T, param_idx, nparam, r, *denom, D, k, dI + k);
   return true;
 }
 
 #if defined(__CUDACC__)
-// One thread per ray; S is the dual numbers' scalar (float: the FP32 DE of the
-// forward; double: FP64 duals, for the central-difference normal's cancellation).
-template <class Set, class S, bool kBatched>
-__global__ void __launch_bounds__(128) adjoint_kernel(const __grid_constant__ AdjointArgs a,
-                                                      const __grid_constant__ DevView single) {
-  const int64_t it = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int K = a.nparam + kPoseParams;
-  double acc[kMaxAdjParams + kPoseParams];
-  for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k) acc[k] = 0.0;
-  int vi = -1;
-  if (it < a.total_rays) {
-    vi = kBatched ? find_view(a.views, a.nviews, it) : 0;
-    const DevView& v = kBatched ? a.views[vi] : single;
-    const int64_t local = it - v.ray_offset;
-    const int64_t r = v.out_offset + local;
-    const float w_loss = a.grad ? a.dL_dshade[r] : 0.0f;
-    double dI[kMaxAdjParams + kPoseParams];
-    for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k) dI[k] = 0.0;
-    if (a.normal4[4 * r + 3] > 0.5f && (w_loss != 0.0f || a.dshade)) {
-      if (adjoint_pixel<Set, S>(v, a.tangents[kBatched ? vi : 0], a.param_idx, a.nparam, local, a.depth64[r], dI)) {
-        for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k)
-          if (k < K) acc[k] = double(w_loss) * dI[k];
-      } else {
-        for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k) dI[k] = 0.0;
-      }
-    }
-    if (a.dshade)
-      for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k)
-        if (k < K) a.dshade[r * K + k] = dI[k];
+// Appends a block's wanted rays to a list: one atomic per block, so that the list keeps
+// runs of neighbouring rays together.  Returns this thread's slot (when it wants one).
+__device__ __forceinline__ unsigned block_append(bool want, unsigned* count) {
+  __shared__ unsigned warp_want[32], base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  __syncthreads();  // the last call's slots have been read
+  if (lane == 0) warp_want[warp] = unsigned(__popc(m));
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned n = 0;
+    for (int w = 0; w < warps; ++w) n += warp_want[w];
+    base = n ? atomicAdd(count, n) : 0u;
   }
-  if (!a.grad) return;
-  // reduce within the warp when every lane has the same view, else per lane
-  const unsigned full = 0xffffffffu;
-  const int uv = vi >= 0 ? (kBatched ? a.views[vi].user_index : single.user_index) : -1;
-  const int uv0 = __shfl_sync(full, uv, 0);
-  const bool uniform = __all_sync(full, uv == uv0);
-  for (int k = 0; k < kMaxAdjParams + kPoseParams; ++k) {
-    if (k >= K) break;
-    double x = acc[k];
-    if (uniform) {
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(full, x, o);
-      if ((threadIdx.x & 31) == 0 && uv0 >= 0 && x != 0.0) atomicAdd(&a.grad[uv0 * K + k], x);
-    } else if (uv >= 0 && x != 0.0) {
-      atomicAdd(&a.grad[uv * K + k], x);
+  __syncthreads();
+  unsigned at = base + __popc(m & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) at += warp_want[w];
+  return at;
+}
+
+// The rays of [first, last) that may contribute (hits with a loss weight, or every hit
+// when the Jacobian is asked for), as indices from first, in hits[0 .. *count).  The
+// Jacobian rows of every ray are zeroed here.
+__global__ static void __launch_bounds__(256) adjoint_list_kernel(const __grid_constant__ AdjointArgs a) {
+  const int64_t it = a.first + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int K = a.nparam + kPoseParams;
+  bool want = false;
+  if (it < a.last) {
+    const DevView& v = a.views[find_view(a.views, a.nviews, it)];
+    const int64_t r = v.out_offset + it - v.ray_offset;
+    want = a.normal4[4 * r + 3] > 0.5f && (a.dshade || a.dL_dshade[r] != 0.0f);
+    if (a.dshade)
+      for (int k = 0; k < K; ++k) a.dshade[r * K + k] = 0.0;
+  }
+  const unsigned at = block_append(want, a.counts);
+  if (want) a.hits[at] = int(it - a.first);
+}
+
+// The adjoint of a listed hit is two kernels.  The first, one lane per hit, does what all
+// thetas share: the DE's value and gradient at the hit and its values at the six normal
+// taps.  About half of the hits end there (back-lit normals).  The second does a lit ray's
+// K = nparam + 3 derivatives, 7 dual evaluations each, C thetas to an evaluation: C = 1
+// for FP32 duals, whose tangents cost as much as their values, 3 for FP64 duals, whose
+// values (64-bit arccosine, powers, sines) are most of an evaluation.  Both lists are
+// dense, so that no lane waits for a neighbour that missed, was back-lit or had no weight:
+// one kernel with one lane per ray of the image and one tangent per evaluation ran with 15
+// (FP32) and 13 (FP64) of 32 lanes active.  The kernels are bound by instruction issue
+// (FP32) and by the FP64 pipe's latency (FP64, 168 registers).  A backward call with two
+// parameters: 4 views of 512 x 512, FP32, 2.10 -> 1.00 ms; 2 views of 256 x 256, FP64,
+// 4.07 -> 0.83 ms.
+template <class Set, class S>
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? kSurfaceBlocks32 : kSurfaceBlocks64)
+    adjoint_surface_kernel(const __grid_constant__ AdjointArgs a) {
+  const int n = int(a.counts[0]);
+  const int stride = int(gridDim.x) * int(blockDim.x);
+  for (int first = int(blockIdx.x) * int(blockDim.x); first < n; first += stride) {  // block-uniform
+    const int entry = first + int(threadIdx.x);
+    bool lit = false;
+    LitRay o;
+    if (entry < n) {
+      const int64_t it = a.first + a.hits[entry];
+      o.ray = int(it - a.first);
+      o.view = find_view(a.views, a.nviews, it);
+      const DevView& v = a.views[o.view];
+      const int64_t local = it - v.ray_offset;
+      double none[kMaxAdjParams + kPoseParams];
+      lit = adjoint_surface<Set, S>(v, a.tangents[o.view], a.param_idx, a.nparam, a.inline_thetas,
+                                    adjoint_ray(v, local, a.depth64[v.out_offset + local]), &o.denom, o.D, none);
+      if (a.inline_thetas > 0) o.denom = none[0];  // never taken: it keeps the loop's results in use
     }
+    const unsigned at = block_append(lit, a.counts + 1);
+    if (lit) a.lit[at] = o;
   }
 }
 
-template <class Set, class S, bool kBatched>
-cudaError_t launch_adjoint(const AdjointArgs& a, const DevView& single, cudaStream_t s) {
-  const int64_t grid = (a.total_rays + 127) / 128;
-  if (grid <= 0) return cudaSuccess;
-  adjoint_kernel<Set, S, kBatched><<<unsigned(grid), 128, 0, s>>>(a, single);
+// One lane per lit ray and chunk of C thetas; the chunks of a ray are
+// neighbours.  A lane keeps its chunk from one ray to the next (the stride is a multiple
+// of the chunks), so it sums its view's gradient in registers.
+template <class Set, class S, int C>
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? kThetaBlocks32 : kThetaBlocks64)
+    adjoint_theta_kernel(const __grid_constant__ AdjointArgs a) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int K = a.nparam + kPoseParams;
+  const int chunks = (K + C - 1) / C;
+  const int64_t items = int64_t(a.counts[1]) * chunks;
+  const int64_t threads = int64_t(gridDim.x) * blockDim.x;
+  const int64_t stride = threads / chunks * chunks;
+  const int64_t me = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int k0 = int(me % chunks) * C;
+  double acc[C];
+  for (int c = 0; c < C; ++c) acc[c] = 0.0;
+  int cur = -1;
+  // adds the sums of the lanes whose view is not `keep`: one atomic per view and theta
+  auto flush = [&](int keep) {
+    unsigned left = __ballot_sync(full, cur >= 0 && cur != keep);
+    while (left) {
+      const int src = __ffs(left) - 1;
+      const int view = __shfl_sync(full, cur, src), k = __shfl_sync(full, k0, src);
+      const bool in = cur == view && k0 == k && cur != keep;
+      left &= ~__ballot_sync(full, in);
+      for (int c = 0; c < C; ++c) {
+        if (k + c >= K) break;
+        double x = in ? acc[c] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(full, x, o);
+        if (lane == 0 && x != 0.0) atomicAdd(&a.grad[int64_t(a.views[view].user_index) * K + k + c], x);
+      }
+      if (in) cur = -1;
+    }
+  };
+  for (int64_t base = me - lane; base < items; base += stride) {  // warp-uniform
+    const int64_t item = base + lane;
+    const bool live = item < items && me < stride;
+    LitRay o;
+    if (live) o = a.lit[item / chunks];
+    if (a.grad) {
+      const int view = live ? o.view : cur;
+      if (__any_sync(full, cur >= 0 && view != cur)) flush(view);
+      if (live && cur < 0) {
+        cur = view;
+        for (int c = 0; c < C; ++c) acc[c] = 0.0;
+      }
+    }
+    if (live) {
+      const DevView& v = a.views[o.view];
+      const int64_t local = a.first + o.ray - v.ray_offset;
+      const int64_t r = v.out_offset + local;
+      double dI[C];
+      adjoint_thetas<Set, S, C>(v, a.tangents[o.view], a.param_idx, a.nparam, adjoint_ray(v, local, a.depth64[r]),
+                                o.denom, D3{o.D[0], o.D[1], o.D[2]}, k0, dI);
+      const double w = a.grad ? double(a.dL_dshade[r]) : 0.0;
+      for (int c = 0; c < C; ++c) {
+        if (k0 + c >= K) break;
+        if (a.dshade) a.dshade[r * K + k0 + c] = dI[c];
+        acc[c] += w * dI[c];
+      }
+    }
+  }
+  if (a.grad) flush(-2);
+}
+
+// A resident grid of a kernel that strides over at most `most` lanes of work.
+template <class Kernel> cudaError_t launch_listed(Kernel kernel, const AdjointArgs& a, int64_t most, cudaStream_t s) {
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
+  if (e != cudaSuccess) return e;
+  const int64_t needed = (most + 127) / 128, resident = int64_t(a.num_sms) * (per_sm < 1 ? 1 : per_sm);
+  kernel<<<unsigned(needed < resident ? needed : resident), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
-typedef cudaError_t (*AdjointFn)(const AdjointArgs&, const DevView&, cudaStream_t);
+template <class Set, class S> cudaError_t launch_adjoint(AdjointArgs a, cudaStream_t s) {
+  constexpr int C = sizeof(S) == 4 ? 1 : 3;
+  const int chunks = (a.nparam + kPoseParams + C - 1) / C;
+  for (a.first = 0; a.first < a.total_rays; a.first = a.last) {
+    a.last = a.total_rays - a.first > kAdjointRays ? a.first + kAdjointRays : a.total_rays;
+    const int64_t n = a.last - a.first;
+    cudaError_t e = cudaMemsetAsync(a.counts, 0, 2 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    adjoint_list_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(a);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_listed(adjoint_surface_kernel<Set, S>, a, n, s);
+    if (e == cudaSuccess) e = launch_listed(adjoint_theta_kernel<Set, S, C>, a, n * chunks, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+typedef cudaError_t (*AdjointFn)(AdjointArgs, cudaStream_t);
 #endif
 
 }  // namespace nd

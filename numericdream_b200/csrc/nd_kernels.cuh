@@ -656,7 +656,7 @@ struct KernelTable {
   LaunchFn inline_f32, inline_f32_batched, inline_f32_dir64, inline_f32_dir64_batched, inline_f64, inline_f64_batched;
   ShadeFn shade_f32, shade_f32_batched, shade_f32_dir64, shade_f32_dir64_batched, shade_f64, shade_f64_batched;
   DePointsFn de_points_f32, de_points_f64;
-  AdjointFn adjoint_f32, adjoint_f32_batched, adjoint_f64, adjoint_f64_batched;
+  AdjointFn adjoint_f32, adjoint_f64;
   // multi-instance scenes (formula groups only; null in single-formula tables)
   LaunchFn scene_persistent_f32, scene_persistent_f32_dir64, scene_persistent_f64;
   ShadeFn scene_shade_f32, scene_shade_f32_dir64, scene_shade_f64;
@@ -754,10 +754,8 @@ template <class Set, bool kWithScenes = false, bool kForwardOnly = false> Kernel
   t.de_points_f32 = &launch_de_points<Set, float>;
   t.de_points_f64 = &launch_de_points<Set, double>;
   if constexpr (!kForwardOnly) {
-    t.adjoint_f32 = &launch_adjoint<Set, float, false>;
-    t.adjoint_f32_batched = &launch_adjoint<Set, float, true>;
-    t.adjoint_f64 = &launch_adjoint<Set, double, false>;
-    t.adjoint_f64_batched = &launch_adjoint<Set, double, true>;
+    t.adjoint_f32 = &launch_adjoint<Set, float>;
+    t.adjoint_f64 = &launch_adjoint<Set, double>;
   }
   return t;
 }

@@ -97,6 +97,8 @@ struct nd_ctx {
   uint64_t last_accel_voxels = 0;
   nd_lite_desc* d_lite = nullptr;    // lite-shading descriptors, in plan order
   int lite_cap = 0;
+  char* d_adjoint = nullptr;         // the adjoint's counters and lists (adjoint_cap rays)
+  int64_t adjoint_cap = 0;
   bool last_trap = false;
   DevView* h_views = nullptr;  // pinned staging: two halves of h_views_cap records, forward calls alternate
   DevView* d_fviews = nullptr;  // the forward's device view table: two halves of fviews_half records, alternating
@@ -1012,6 +1014,7 @@ nd_status nd_ctx_destroy(nd_ctx* ctx) {
   if (ctx->d_accel) cudaFree(ctx->d_accel);
   if (ctx->d_accel_jobs) cudaFree(ctx->d_accel_jobs);
   if (ctx->d_lite) cudaFree(ctx->d_lite);
+  if (ctx->d_adjoint) cudaFree(ctx->d_adjoint);
   for (int k = 0; k < 2; ++k)
     if (ctx->staged[k]) {
       if (ctx->staged_valid[k]) cudaEventSynchronize(ctx->staged[k]);
@@ -2207,6 +2210,16 @@ extern "C" nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, c
   }
   DevView* dv = nullptr;
   nd::PoseTangents* dt = nullptr;
+  // scratch of the context: the call waits for its work, so calls never share it
+  const int64_t listed = std::min(total, nd::kAdjointRays);
+  if (ctx->adjoint_cap < listed) {
+    if (ctx->d_adjoint) cudaFree(ctx->d_adjoint);
+    ctx->d_adjoint = nullptr;
+    ctx->adjoint_cap = 0;
+    e = cudaMalloc((void**)&ctx->d_adjoint, 256 + size_t(listed) * (sizeof(nd::LitRay) + sizeof(int32_t)));
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint lists");
+    ctx->adjoint_cap = listed;
+  }
   e = cudaMallocAsync((void**)&dv, sizeof(DevView) * hv.size(), st);
   if (e == cudaSuccess) e = cudaMallocAsync((void**)&dt, sizeof(nd::PoseTangents) * ht.size(), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dv, hv.data(), sizeof(DevView) * hv.size(), cudaMemcpyHostToDevice, st);
@@ -2229,13 +2242,16 @@ extern "C" nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, c
     a.nparam = nparams;
     for (int k = 0; k < nparams; ++k) a.param_idx[k] = param_idx[k];
     const KernelTable& kt = plans[p].table;
-    const nd::AdjointFn fn = prec == 64 ? (nv > 1 ? kt.adjoint_f64_batched : kt.adjoint_f64)
-                                        : (nv > 1 ? kt.adjoint_f32_batched : kt.adjoint_f32);
+    const nd::AdjointFn fn = prec == 64 ? kt.adjoint_f64 : kt.adjoint_f32;
     if (!fn) {
       e = cudaErrorNotSupported;
       break;
     }
-    e = fn(a, hv[first[p]], st);
+    a.num_sms = ctx->num_sms;
+    a.counts = reinterpret_cast<unsigned*>(ctx->d_adjoint);
+    a.lit = reinterpret_cast<nd::LitRay*>(ctx->d_adjoint + 256);
+    a.hits = reinterpret_cast<int32_t*>(a.lit + ctx->adjoint_cap);
+    e = fn(a, st);
   }
   // the host staging vectors are pageable: wait for the copies before they go away
   cudaError_t e2 = cudaStreamSynchronize(st);

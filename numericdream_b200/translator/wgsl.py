@@ -598,6 +598,7 @@ F32, I32, U32, BOOL, AINT, AFLOAT = S("f32"), S("i32"), S("u32"), S("bool"), S("
 VOID = Ty("void")
 PARAMS = Ty("params")
 CARRY = Ty("st", name="IterCarry")
+MUL_ANGLE = Ty("st", name="MulAngle")  # translator-made: an acos or atan2 times a factor
 IMAGE_INFO = Ty("st", name="ImageInfo")
 IMAGE_SAMPLE = Ty("st", name="ImageSample")
 # struct types a formula may use: its carry, and the image sampler's records
@@ -1422,6 +1423,8 @@ class FormulaCompiler:
                     return x.ty
             return xs[0].ty
 
+        if name in ("sin", "cos") and len(args) == 1 and args[0].ty == MUL_ANGLE:
+            return TE(F32, f"ndw::{name}_of({args[0].code})")
         if name in _FLOAT_UNARY:
             (a,) = float_args(args, 1)
             if a.ty.scalar != "f32":
@@ -1552,6 +1555,11 @@ class FormulaCompiler:
                 return ""
             # a const bound to a non-constant expression is a let
         ty = self.resolve_type(s.ty) if s.ty is not None else None
+        angle = self.mul_angle(s)
+        if angle is not None:
+            cname = cpp_name(s.name)
+            self.declare(s.name, TE(MUL_ANGLE, cname, None, lvalue=False), s.line)
+            return f"const ndw::MulAngle<T> {cname} = {angle};"
         if s.init is not None:
             te = self.expr(s.init)
             if ty is None:
@@ -1570,6 +1578,34 @@ class FormulaCompiler:
         if init is None:
             return f"{qual}{cpp_type(ty)} {cname}{{}};"
         return f"{qual}{cpp_type(ty)} {cname} = {init};"
+
+    def mul_angle(self, s: Decl):
+        """`let a = acos(x) * f;` (or atan2(y, x) * f) whose every use is sin(a) or cos(a):
+        ndw::MulAngle may hold its sine and cosine in place of the angle.  Returns the
+        initialiser's code, None for any other declaration."""
+        e = s.init
+        if (s.kind != "let" or not isinstance(e, Binary) or e.op != "*" or not isinstance(e.l, Call) or
+                (e.l.name, len(e.l.args)) not in (("acos", 1), ("atan2", 2)) or e.l.name in self.fn_sigs or
+                "sin" in self.fn_sigs or "cos" in self.fn_sigs or self.helper_ns != "ndw" or
+                (s.ty is not None and self.resolve_type(s.ty) != F32)):
+            return None
+        body = self.fns[self.cur_fn].body
+        decls, uses, in_trig = 0, 0, 0
+        for node in walk_nodes([body, [p[0] for p in self.fns[self.cur_fn].params]]):
+            if isinstance(node, Decl) and node.name == s.name or node == s.name:
+                decls += 1
+            elif isinstance(node, Ident) and node.name == s.name:
+                uses += 1
+            elif (isinstance(node, Call) and node.name in ("sin", "cos") and len(node.args) == 1 and
+                  isinstance(node.args[0], Ident) and node.args[0].name == s.name):
+                in_trig += 1
+        if decls != 1 or uses != in_trig:
+            return None
+        args = [self.expr(a) for a in e.l.args]
+        factor = self.expr(e.r)
+        if any(te.ty != F32 for te in args + [factor]):
+            return None
+        return f"ndw::{e.l.name}_times({', '.join(te.code for te in args + [factor])})"
 
     def assign_code(self, s: Assign) -> str:
         lhs = self.expr(s.lhs)
@@ -1825,6 +1861,21 @@ class FormulaCompiler:
                 lines.append("}")
         lines.append(f"}}  // namespace {self.ns}")
         return "\n".join(lines)
+
+
+def walk_nodes(x):
+    """Every syntax node (and plain string) under x, depth first."""
+    if isinstance(x, (list, tuple)):
+        for y in x:
+            yield from walk_nodes(y)
+    elif dataclasses.is_dataclass(x):
+        yield x
+        for f in dataclasses.fields(x):
+            v = getattr(x, f.name)
+            if isinstance(v, (list, tuple)) or dataclasses.is_dataclass(v):
+                yield from walk_nodes(v)
+    elif isinstance(x, str):
+        yield x
 
 
 @dataclasses.dataclass

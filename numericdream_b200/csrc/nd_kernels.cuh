@@ -121,14 +121,22 @@ __global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::valu
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  Lane<T, kDir64> L;
+  typename std::conditional<kDefer, MarchLane<T, kDir64>, Lane<T, kDir64>>::type L;
   L.item = -1;
   L.view = 0;
-  L.phase = PH_DONE;
-  L.evals = 0;
   L.hit = false;
-  L.lazy = true;
-  L.pending = 0;
+  if constexpr (kDefer) {
+    L.mode = L.kDone;
+  } else {
+    L.phase = PH_DONE;
+    L.evals = 0;
+    L.lazy = true;
+    L.pending = false;
+  }
+  auto done = [&]() {
+    if constexpr (kDefer) return L.mode == L.kDone;
+    else return L.phase == PH_DONE;
+  };
   uint32_t rays = 0, hits = 0, ev_m = 0, ev_n = 0, ev_s = 0, refills = 0;
   const int64_t deadline = __shfl_sync(full, globaltimer_ns(), 0) + a.deadline_ns;
   int tick = 0;
@@ -139,20 +147,15 @@ __global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::valu
   // Finished rays keep their lane until the next refill: their outputs are written
   // then, all together, instead of in the pass that ends each ray.
   auto retire = [&]() {
-    int32_t hit_item = -1;
-    uint32_t hit_evals = 0;
-    double hit_t = 0.0;
-    if (L.item >= 0 && L.phase == PH_DONE) {
+    HitEntry hit;
+    hit.item = -1;
+    if (L.item >= 0 && done()) {
       const DevView& v = kBatched ? a.views[L.view] : single;
       if constexpr (kDefer) {
-        // the hit distance travels in the hit list: no per-ray distance array
-        L.flush_deferred(v, a.out, nullptr);
-        ev_m += L.evals;
-        if (L.hit) {
-          hit_item = L.item;
-          hit_evals = L.evals;
-          hit_t = L.t;
-        }
+        const uint32_t evals = L.evals(v);
+        ev_m += evals;
+        if (L.hit) hit = HitEntry{L.item, L.i, evals, 0, L.a, L.st};
+        else write_miss(v, a.out, v.out_offset + (int64_t(L.item) - v.ray_offset), evals);
       } else {
         L.flush(v, a.out, a.t_hit);
         const uint32_t taps = L.hit ? normal_taps(v) : 0u;
@@ -166,18 +169,18 @@ __global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::valu
     }
     if constexpr (defer) {
       // append the retired hits to the shade pass's list, one atomic per warp
-      const unsigned hm = __ballot_sync(full, hit_item >= 0);
+      const unsigned hm = __ballot_sync(full, hit.item >= 0);
       if (hm) {
         unsigned base = 0;
         if (lane == 0) base = atomicAdd(a.hit_count, unsigned(__popc(hm)));
         base = __shfl_sync(full, base, 0);
-        if (hit_item >= 0) a.hit_list[base + __popc(hm & lt_mask)] = HitEntry{hit_item, hit_evals, hit_t};
+        if (hit.item >= 0) a.hit_list[base + __popc(hm & lt_mask)] = hit;
       }
     }
   };
   while (true) {
-    // an idle lane (item < 0) is always in PH_DONE, so phase alone tells busy lanes
-    const unsigned free_lanes = __ballot_sync(full, L.phase == PH_DONE);
+    // an idle lane (item < 0) is always done, so that alone tells the busy lanes
+    const unsigned free_lanes = __ballot_sync(full, done());
     const int nfree = __popc(free_lanes);
     const bool have_work = runs.have_work();
     if (!have_work && free_lanes == full) {
@@ -199,8 +202,12 @@ __global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::valu
           const int32_t it = c.item(r);
           L.view = kBatched ? find_view_from(a.views, a.nviews, it, L.view) : 0;
           const DevView& v = kBatched ? a.views[L.view] : single;
-          L.start(v, it, L.view, true);
-          if (L.phase == PH_DONE) L.finish(v, a.out, a.t_hit, 1.0f);
+          if constexpr (kDefer) {
+            L.start(v, it, L.view);
+          } else {
+            L.start(v, it, L.view, true);
+            if (L.phase == PH_DONE) L.finish(v, a.out, a.t_hit, 1.0f);
+          }
         }
       }
       continue;  // lanes that finished at once go back through the bookkeeping
@@ -214,18 +221,20 @@ __global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::valu
         break;
       }
     }
-    if (L.phase != PH_DONE) {
+    if (!done()) {
       const DevView& v = kBatched ? a.views[L.view] : single;
-      bool probe = true;
-      if constexpr (kAccel) {
-        // the accelerator's jumps come before the probe; a ray with more jumps to take
-        // than the per-pass limit takes the rest in later passes
-        if (L.phase == PH_MARCH && L.probing && v.accel_levels > 0)
-          probe = L.accel_skips(v, a.out, a.t_hit, a.accel_chain);
-      }
-      if (probe && L.phase != PH_DONE) {
+      if constexpr (kDefer) {
+        bool probe = true;
+        if constexpr (kAccel) {
+          // the accelerator's jumps come before the probe; a ray with more jumps to take
+          // than the per-pass limit takes the rest in later passes
+          if ((L.mode == L.kProbe || L.mode == L.kVerify) && v.accel_levels > 0)
+            probe = L.accel_skips(v, a.accel_chain);
+        }
+        if (probe) L.advance(v, view_de<Set, T, false, kScenes>(v, to_t<T>(L.sample_pos(v)), a.scenes).d);
+      } else {
         const DEOut<T> de = view_de<Set, T, false, kScenes>(v, to_t<T>(L.sample_pos(v)), a.scenes);
-        L.template advance<kDefer>(v, de, a.out, a.t_hit, kDefer);
+        L.advance(v, de, a.out, a.t_hit);
       }
     }
   }
@@ -256,26 +265,40 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
   const bool queue = a.shadow_queue != nullptr;
   const int64_t count = list ? int64_t(*a.hit_count) : a.total_rays;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  unsigned long long taps = 0, shadow = 0;
+  uint32_t taps = 0, shadow = 0, bisect = 0, lost = 0;
   for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); i0 < count; i0 += stride) {
     const int64_t i = i0 + lane;  // the loop bound is warp-uniform: every lane takes part in the ballot
     bool want = false;
     ShadowEntry e;
     if (i < count) {
-      HitEntry h{int32_t(i), 0u, 0.0};
+      HitEntry h{int32_t(i), 0, 0u, 0, 0.0, 0.0};
       if (list) h = a.hit_list[i];
       const int64_t it = h.item;
       const int vi = kBatched ? find_view(a.views, a.nviews, it) : 0;
       const DevView& v = kBatched ? a.views[vi] : single;
       const int64_t local = it - v.ray_offset;
       const int64_t r = v.out_offset + local;
-      const double t = list ? h.t : a.t_hit[r];
+      double t = list ? h.b : a.t_hit[r];
       if (t >= 0.0) {  // (all-rays mode: a miss has t < 0 and the march wrote its outputs)
-        // one call site per kind of DE evaluation (normal taps, shadow steps, trap), so
-        // that the formula set's code appears three times in the kernel
+        // one call site per kind of DE evaluation (bisection, normal taps, shadow steps,
+        // trap), so that the formula set's code appears four times in the kernel
         Dir<kDir64> dir;
         dir.set(ray_dir(v, local));
+        bool hit = true;
         if (list) {
+          int used = 0;
+          hit = resolve_hit<Set, T, kDir64, kScenes>(v, dir, h, a.scenes, &t, &used);
+          bisect += uint32_t(used);
+          h.evals += uint32_t(used);
+          if (!hit) {
+            ++lost;
+            write_miss(v, a.out, r, h.evals);
+          }
+        }
+        if (list && hit) {
+          a.out.depth[r] = float(t);
+          if (a.out.steps) a.out.steps[r] = uint32_t(h.steps);
+          if (a.out.depth64) a.out.depth64[r] = t;
           const Surface sf = surface_at_hit<Set, T, kDir64, kScenes>(v, dir, t, r, a.out, a.scenes);
           taps += uint32_t(sf.taps);
           float vis = 1.0f;
@@ -283,7 +306,7 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
           if (casts_shadow(v)) {
             const D3 so = shadow_origin(sf);
             if (queue) {
-              e = ShadowEntry{h.item, h.march_evals + uint32_t(sf.taps), sf.gx, sf.gy, sf.gz, 0, so.x, so.y, so.z};
+              e = ShadowEntry{h.item, h.evals + uint32_t(sf.taps), sf.gx, sf.gy, sf.gz, 0, so.x, so.y, so.z};
               want = true;
             } else {
               vis = shadow_visibility<Set, T, kScenes, kAccel>(v, so, a.scenes, &sev);
@@ -291,9 +314,9 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
             }
           }
           if (!want)
-            finish_at_hit(v, dir.get(), sf.gx, sf.gy, sf.gz, vis, h.march_evals + uint32_t(sf.taps + sev), r, a.out);
+            finish_at_hit(v, dir.get(), sf.gx, sf.gy, sf.gz, vis, h.evals + uint32_t(sf.taps + sev), r, a.out);
         }
-        if (do_trap)
+        if (do_trap && hit)
           trap_at_point<Set, T, kScenes>(v, fmadd(d3(v.org[0], v.org[1], v.org[2]), dir.get(), t), r, a.out,
                                          a.scenes);
       }
@@ -312,12 +335,16 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
     for (int o = 16; o > 0; o >>= 1) {
       taps += __shfl_xor_sync(full, taps, o);
       shadow += __shfl_xor_sync(full, shadow, o);
+      bisect += __shfl_xor_sync(full, bisect, o);
+      lost += __shfl_xor_sync(full, lost, o);
     }
-    if (lane == 0 && taps + shadow) {
-      atomicAdd(&a.stats->normal_evals, taps);
-      atomicAdd(&a.stats->shadow_evals, shadow);
-      atomicAdd(&a.stats->de_evals, taps + shadow);
+    if (lane == 0 && taps + shadow + bisect) {
+      atomicAdd(&a.stats->normal_evals, (unsigned long long)taps);
+      atomicAdd(&a.stats->shadow_evals, (unsigned long long)shadow);
+      atomicAdd(&a.stats->march_evals, (unsigned long long)bisect);
+      atomicAdd(&a.stats->de_evals, (unsigned long long)taps + shadow + bisect);
     }
+    if (lane == 0 && lost) atomicAdd(&a.stats->hits, 0ull - lost);
   }
 }
 

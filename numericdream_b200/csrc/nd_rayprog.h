@@ -46,6 +46,7 @@ ND_DEV_INLINE double rn_add(double a, double b) { return __dadd_rn(a, b); }
 ND_DEV_INLINE double fma_d(double a, double b, double c) { return __fma_rn(a, b, c); }
 ND_DEV_INLINE float load_ro(const float* p) { return __ldg(p); }
 ND_DEV_INLINE int32_t float_bits(float x) { return __float_as_int(x); }
+ND_DEV_INLINE uint32_t low_word(double x) { return uint32_t(__double2loint(x)); }
 ND_DEV_INLINE uint16_t half_bits(float x) { return __half_as_ushort(__float2half_rn(x)); }
 #else
 // host builds of this header are compiled with -ffp-contract=off
@@ -59,6 +60,11 @@ ND_DEV_INLINE int32_t float_bits(float x) {
   int32_t b;
   memcpy(&b, &x, sizeof(b));
   return b;
+}
+ND_DEV_INLINE uint32_t low_word(double x) {
+  uint64_t b;
+  memcpy(&b, &x, sizeof(b));
+  return uint32_t(b);
 }
 // IEEE binary16 bits of x, rounded to nearest even (host builds of the ray program)
 ND_DEV_INLINE uint16_t half_bits(float x) {
@@ -125,6 +131,7 @@ struct DevView {
   float accel_cam[3];   // the camera position the cascades are centred on (f32)
   float accel_k;        // 1 / ((res / 2 - 1) * finest cell): lookup start level
   ndw::ImageRef image;  // the formula image (texels nullptr: none)
+  double inv_width, inv_height;  // 1 / width, 1 / height (div_known)
   // n / d for 0 <= n < 2^31 as (n * m) >> s (DivMagic): d = the tile's pixels, d = its width
   uint32_t npix_m, npix_s, width_m, width_s;
 };
@@ -143,19 +150,49 @@ ND_DEV_INLINE void div_magic(uint32_t d, uint32_t* m, uint32_t* s) {
 }
 ND_DEV_INLINE uint32_t div_by(uint32_t n, uint32_t m, uint32_t s) { return uint32_t((uint64_t(n) * m) >> s); }
 
+// a / b, correctly rounded, for a divisor b whose reciprocal y (correctly rounded) is
+// known: two corrections of a * y by the exact remainder (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).  Five FP64
+// operations in a straight line; a 64-bit division is several times that, with a branch.
+// For finite a and b well inside the exponent range (pixel coordinates here).
+ND_DEV_INLINE double div_known(double a, double b, double y) {
+  const double q0 = rn_mul(a, y);
+  const double q1 = fma_d(fma_d(-q0, b, a), y, q0);
+  return fma_d(fma_d(-q1, b, a), y, q1);
+}
+
+// 1 / sqrt(s) with both operations correctly rounded, from y, an approximation of it to
+// about an ulp: the same corrections, first for the root, then for its reciprocal (whose
+// one exception, a divisor of all ones, divides).
+ND_DEV_INLINE double inv_sqrt_from(double s, double y) {
+  const double g0 = rn_mul(s, y);
+  const double g = fma_d(fma_d(-g0, g0, s), 0.5 * y, g0);
+  if (low_word(g) == 0xffffffffu) return 1.0 / g;
+  const double y1 = fma_d(fma_d(-g, y, 1.0), y, y);
+  return fma_d(fma_d(-g, y1, 1.0), y1, y1);
+}
+ND_DEV_INLINE double inv_sqrt(double s) {
+#if defined(__CUDA_ARCH__)
+  if (s > 1e-200 && s < 1e200) return inv_sqrt_from(s, ::rsqrt(s));
+#endif
+  return 1.0 / sqrt(s);
+}
+
 struct Stats {
   unsigned long long rays, de_evals, march_evals, normal_evals, shadow_evals, hits, refills;
   unsigned int timeouts, pad;
 };
 
-// One entry of the deferred shade pass's hit list: the launch-local ray index, the DE
-// evaluations its march used (the shade pass writes the ray's total once) and the FP64
-// hit distance.  The surface pass reads its hits in list order, 16 B each and
-// coalesced, instead of fetching each hit's distance from a per-ray array.
+// One entry of the deferred march's hit list: the launch-local ray index, the probe steps
+// and DE evaluations its march used, and the bracket of the hit: the distance of the last
+// sample above eps and of the first below it (both the hit itself when nothing is left
+// to bisect).  The surface pass reads its hits in list order, 32 B each and coalesced.
 struct HitEntry {
   int32_t item;
-  uint32_t march_evals;
-  double t;
+  int32_t steps;
+  uint32_t evals;
+  int32_t pad;
+  double a, b;
 };
 
 // One entry of the shadow queue (the wavefront shadow pass, after cs_wf_shadow
@@ -662,8 +699,8 @@ ND_DEV_INLINE void ray_uv(const DevView& v, int64_t local, double* ux, double* u
     jx = double(uint32_t(h) >> 8) * (1.0 / 16777216.0);
     jy = double(uint32_t(h >> 32) >> 8) * (1.0 / 16777216.0);
   }
-  const double ndc_x = 2.0 * (double(px) + jx) / double(v.width) - 1.0;
-  const double ndc_y = 1.0 - 2.0 * (double(py) + jy) / double(v.height);
+  const double ndc_x = div_known(2.0 * (double(px) + jx), double(v.width), v.inv_width) - 1.0;
+  const double ndc_y = 1.0 - div_known(2.0 * (double(py) + jy), double(v.height), v.inv_height);
   *ux = ndc_x * v.aspect;
   *uy = -ndc_y;
 }
@@ -674,7 +711,7 @@ ND_DEV_INLINE D3 ray_dir(const DevView& v, int64_t local) {
   double x = v.fwd[0] + v.right[0] * ux + v.up[0] * uy;
   double y = v.fwd[1] + v.right[1] * ux + v.up[1] * uy;
   double z = v.fwd[2] + v.right[2] * ux + v.up[2] * uy;
-  const double inv = 1.0 / sqrt(x * x + y * y + z * z);
+  const double inv = inv_sqrt(x * x + y * y + z * z);
   return D3{x * inv, y * inv, z * inv};
 }
 
@@ -878,12 +915,12 @@ template <class T, bool kDir64> struct Lane {
   uint32_t mev;   // evaluations the march used (set when the march ends)
   bool probing, bisecting, resolved, hit;
   bool lazy;        // outputs wait for flush() (the persistent kernel writes them in batches)
-  uint8_t pending;  // outputs not yet written: 1 finish's, 2 finish_march's
+  bool pending;     // finish's outputs are not yet written
   float vis;        // shadow visibility of a pending finish
 
   ND_DEV_INLINE void start(const DevView& v, int32_t it, int32_t vidx, bool lazy_outputs = false) {
     lazy = lazy_outputs;
-    pending = 0;
+    pending = false;
     item = it;
     view = vidx;
     dir.set(ray_dir(v, int64_t(it) - v.ray_offset));
@@ -909,35 +946,11 @@ template <class T, bool kDir64> struct Lane {
     return fmadd(so, d3(v.light[0], v.light[1], v.light[2]), a);
   }
 
-  // The accelerator's jumps before a probe (march_to tpl:1890-1900): while the
-  // recorded skip at the probe position exceeds eps(t), advance without a DE
-  // evaluation; each jump is a step and a sample of march_to's loop.  May end the
-  // ray (a miss).
-  // At most `chain` jumps (0: no limit); returns true when the ray may probe now,
-  // false when it ended or has more jumps to take (in a later pass).
-  ND_DEV_INLINE bool accel_skips(const DevView& v, const nd_gbuffer& g, double* t_hit, int chain) {
-    const D3 o = d3(v.org[0], v.org[1], v.org[2]);
-    for (int jumps = 0;; ++jumps) {
-      const D3 p = fmadd(o, dir.get(), t);
-      const double skip = double(accel_skip(v, float(p.x), float(p.y), float(p.z)));
-      if (!(skip > march_eps<T>(v, t))) return true;
-      if (chain > 0 && jumps >= chain) return false;
-      a = t;
-      t = t + skip;
-      ++i;
-      ++n;
-      if (t > v.max_dist || i >= v.max_steps || n >= v.max_samples) {
-        finish(v, g, t_hit, 1.0f);
-        return false;
-      }
-    }
-  }
-
   ND_DEV_INLINE void finish(const DevView& v, const nd_gbuffer& g, double* t_hit, float visibility) {
     if (!hit) mev = evals;
     phase = PH_DONE;
     if (lazy) {
-      pending = 1;
+      pending = true;
       vis = visibility;
       return;
     }
@@ -960,30 +973,8 @@ template <class T, bool kDir64> struct Lane {
 
   // Write the outputs a lazy lane left pending.
   ND_DEV_INLINE void flush(const DevView& v, const nd_gbuffer& g, double* t_hit) {
-    if (pending == 1) write_finish(v, g, t_hit, vis);
-    else if (pending == 2) write_march(v, g, t_hit);
-    pending = 0;
-  }
-
-  // The outputs of a miss (write_finish with hit = false and visibility 1).
-  ND_DEV_INLINE void write_miss(const DevView& v, const nd_gbuffer& g, double* t_hit) const {
-    RayResult r;
-    r.hit = false;
-    r.t = t;
-    r.steps = uint32_t(v.max_steps);
-    r.evals = evals;
-    r.nx = r.ny = r.nz = 0.0f;
-    r.shadow = 1.0f;
-    r.shade = 0.0f;
-    write_result(g, t_hit, v.out_offset + (int64_t(item) - v.ray_offset), r);
-  }
-
-  // flush for a march that defers all shading (advance<true>): a lane that finished
-  // without a hit is a miss, one with a hit waits for the surface pass.
-  ND_DEV_INLINE void flush_deferred(const DevView& v, const nd_gbuffer& g, double* t_hit) {
-    if (pending == 1) write_miss(v, g, t_hit);
-    else if (pending == 2) write_march(v, g, t_hit);
-    pending = 0;
+    if (pending) write_finish(v, g, t_hit, vis);
+    pending = false;
   }
 
   ND_DEV_INLINE void begin_normal(double at) {
@@ -995,49 +986,11 @@ template <class T, bool kDir64> struct Lane {
     gx = gy = gz = 0.0f;
   }
 
-  // Deferred shading: a hit ends here with the march's outputs (depth, FP64 t,
-  // steps, evaluations); the shade pass writes normal, shade and shadow.
-  ND_DEV_INLINE void finish_march(const DevView& v, const nd_gbuffer& g, double* t_hit) {
-    phase = PH_DONE;
-    if (lazy) {
-      pending = 2;
-      return;
-    }
-    write_march(v, g, t_hit);
-  }
-
-  // (the evaluation count goes to the shade pass with the hit, which writes the total)
-  ND_DEV_INLINE void write_march(const DevView& v, const nd_gbuffer& g, double* t_hit) const {
-    const int64_t r = v.out_offset + (int64_t(item) - v.ray_offset);
-    g.depth[r] = float(t);
-    if (t_hit) t_hit[r] = t;
-    if (g.steps) g.steps[r] = uint32_t(i);
-    if (g.depth64) g.depth64[r] = t;
-  }
-
-  template <bool kDeferOnly>
-  ND_DEV_INLINE void hit_at(const DevView& v, double at, const nd_gbuffer& g, double* t_hit, bool defer) {
-    if constexpr (kDeferOnly) {
-      // the ray ends at its hit; the normal and shadow phases are the surface pass's
-      t = at;
-      hit = true;
-      finish_march(v, g, t_hit);
-    } else {
-      begin_normal(at);
-      if (defer) finish_march(v, g, t_hit);
-    }
-  }
-
   // Consume one DE result; sets phase = PH_DONE (outputs written) when finished.
-  // With defer_shade a hit ends the ray (finish_march) instead of entering PH_NORMAL.
-  // kDeferOnly: a march that always defers its shading (every lane is in PH_MARCH or
-  // done), compiled without the normal and shadow phases.
-  template <bool kDeferOnly = false>
-  ND_DEV_INLINE void advance(const DevView& v, const DEOut<T>& de, const nd_gbuffer& g, double* t_hit,
-                             bool defer_shade = false) {
+  ND_DEV_INLINE void advance(const DevView& v, const DEOut<T>& de, const nd_gbuffer& g, double* t_hit) {
     ++evals;
     const double d = double(de.d);
-    if (kDeferOnly || phase == PH_MARCH) {
+    if (phase == PH_MARCH) {
       // one pass of march_to's sample loop (tpl:1881-1960); a = lo, b = hi
       const bool on_hit = v.verify == 0;
       const int refine_budget = on_hit ? 0 : v.refine;
@@ -1053,7 +1006,7 @@ template <class T, bool kDir64> struct Lane {
           a = st;
         }
         ++k;
-        if ((b - a <= e && !v.exact_hit) || k >= bisect_budget) hit_at<kDeferOnly>(v, b, g, t_hit, defer_shade);
+        if ((b - a <= e && !v.exact_hit) || k >= bisect_budget) begin_normal(b);
         else if (n >= v.max_samples) finish(v, g, t_hit, 1.0f);  // march_to's loop ran out: a miss
         return;
       }
@@ -1066,7 +1019,7 @@ template <class T, bool kDir64> struct Lane {
           if (n >= v.max_samples) finish(v, g, t_hit, 1.0f);
           return;
         }
-        hit_at<kDeferOnly>(v, st, g, t_hit, defer_shade);
+        begin_normal(st);
         return;
       }
       if (probing && on_hit) {
@@ -1103,7 +1056,6 @@ template <class T, bool kDir64> struct Lane {
       if (n >= v.max_samples) finish(v, g, t_hit, 1.0f);
       return;
     }
-    if constexpr (kDeferOnly) return;
     if (phase == PH_NORMAL) {
       normal_accumulate(v, k, d, gx, gy, gz);
       ++k;
@@ -1133,9 +1085,223 @@ template <class T, bool kDir64> struct Lane {
   }
 };
 
+// --------------------------------------------------------------- the deferred march
+// The ray program of a march that leaves its hits to the surface pass: march_to's probes
+// (tpl:1859-1963), sample for sample as Lane::advance takes them, up to the sample that
+// goes below eps.  Every pass of the march issues this code for a whole warp, so the
+// plain probe of a view that bisects its hits (march_verify off) comes first and is
+// short: one compare, one add, two limits.  What differs from Lane:
+//   st is the distance of the next sample (Lane's t while probing, the bracket's middle
+//   while a verified step is refined), so nothing is selected when a position is formed;
+//   the bisection of a hit is the surface pass's (resolve_hit): there every lane bisects,
+//   while in a warp of the march a few lanes did, in nearly every pass.  With an FP64 DE
+//   only a bisection that runs its whole budget (exact_hit) goes there: the bookkeeping of
+//   a short one is small beside an FP64 evaluation, and the lanes of the surface pass
+//   would wait for the longest of theirs.  Both measured: 64 views, FP32, march and surface
+//   pass 2898 + 521 us with the bisection in the march, 2508 + 651 without; FP64, two views
+//   of 40 exact bisections 3719 + 146 and 2590 + 1044, a close-up that stops at eps 5231 +
+//   719 and 5123 + 1354;
+//   i counts the probes and k the samples after them (the one below eps, the bisection's),
+//   so a view that bisects has taken i + k samples, and while probing the limit on the
+//   samples is not below the one on the steps; n counts a verified march's samples.
+template <class T, bool kDir64> struct MarchLane {
+  enum : int32_t { kProbe, kBisect, kVerify, kRefine, kDone };
+  static constexpr bool kBisects = sizeof(T) == 8;
+  int32_t item;  // work-item index inside the launch, -1 when idle
+  int32_t view;
+  int32_t mode;
+  Dir<kDir64> dir;
+  double st, a, b;
+  int32_t i, k, n;
+  uint32_t jumped;  // accelerator jumps (samples without an evaluation)
+  bool hit;
+
+  ND_DEV_INLINE void start(const DevView& v, int32_t it, int32_t vidx) {
+    item = it;
+    view = vidx;
+    dir.set(ray_dir(v, int64_t(it) - v.ray_offset));
+    st = a = b = 0.0;
+    i = k = n = 0;
+    jumped = 0;
+    hit = false;
+    mode = v.max_samples <= 0 ? kDone : (v.verify == 0 ? kProbe : kVerify);  // no samples: a miss
+  }
+
+  ND_DEV_INLINE D3 sample_pos(const DevView& v) const {
+    return fmadd(d3(v.org[0], v.org[1], v.org[2]), dir.get(), st);
+  }
+  // DE evaluations so far
+  ND_DEV_INLINE uint32_t evals(const DevView& v) const {
+    return uint32_t(v.verify == 0 ? i + k : n) - jumped;
+  }
+
+  // The accelerator's jumps before a probe (march_to tpl:1890-1900): while the
+  // recorded skip at the probe position exceeds eps(t), advance without a DE
+  // evaluation; each jump is a step and a sample of march_to's loop.  May end the
+  // ray (a miss).
+  // At most `chain` jumps (0: no limit); returns true when the ray may probe now,
+  // false when it ended or has more jumps to take (in a later pass).
+  ND_DEV_INLINE bool accel_skips(const DevView& v, int chain) {
+    for (int jumps = 0;; ++jumps) {
+      const D3 p = sample_pos(v);
+      const double skip = double(accel_skip(v, float(p.x), float(p.y), float(p.z)));
+      if (!(skip > march_eps<T>(v, st))) return true;
+      if (chain > 0 && jumps >= chain) return false;
+      a = st;
+      st = st + skip;
+      ++i;
+      ++n;
+      ++jumped;
+      if (st > v.max_dist || i >= v.max_steps || (v.verify != 0 && n >= v.max_samples)) {
+        mode = kDone;
+        return false;
+      }
+    }
+  }
+
+  // Consume one DE result.
+  ND_DEV_INLINE void advance(const DevView& v, T de) {
+    const double d = double(de);
+    const bool below = below_eps<T>(de, d, v, st);
+    if (mode == kProbe && !below) {
+      a = st;
+      st = st + d;
+      ++i;
+      if (st > v.max_dist || i >= v.max_steps) mode = kDone;
+      return;
+    }
+    if (mode >= kVerify) {
+      ++n;
+      if (!below) {
+        verify(v, d);
+        return;
+      }
+      a = st;  // a verified hit is not bisected
+    } else if (kBisects && bisect(v, below)) {
+      return;
+    } else {
+      k += mode == kProbe ? 1 : 0;
+    }
+    hit = true;
+    mode = kDone;
+  }
+
+  // One sample of a bisection, or the sample below eps that starts it.  False: the ray is
+  // at its hit, with the bracket [a, st] as far as it goes.
+  ND_DEV_INLINE bool bisect(const DevView& v, bool below) {
+    if (mode == kProbe) {
+      if (v.exact_hit || !(v.refine > 0 && st - a > march_eps<T>(v, st))) return false;
+      b = st;
+      mode = kBisect;
+    } else {
+      const double e = march_eps<T>(v, st);
+      if (below) b = st;
+      else a = st;
+      if (b - a <= e || k >= v.refine) {
+        ++k;
+        a = st = b;
+        return false;
+      }
+    }
+    ++k;
+    if (i + k >= v.max_samples) mode = kDone;  // march_to's loop ran out: a miss
+    else st = 0.5 * (a + b);
+    return true;
+  }
+
+  // A verified march (march_verify): a probe's step is refined until a sample's DE
+  // covers the rest of it.
+  ND_DEV_INLINE void verify(const DevView& v, double d) {
+    bool resolved = false;
+    if (mode == kVerify) {
+      a = st;
+      b = st + d;
+      k = 0;
+      mode = kRefine;
+    } else {
+      if (d >= b - st) resolved = true;
+      else b = st;
+      ++k;
+    }
+    if (resolved || k >= v.refine) {
+      if (v.hq && !resolved && v.refine > 0) b = fmin(b, a + fmax(a, 1.0) * v.footprint);
+      st = b;
+      ++i;
+      if (st > v.max_dist || i >= v.max_steps) {
+        mode = kDone;
+        return;
+      }
+      mode = kVerify;
+    } else {
+      st = 0.5 * (a + b);
+    }
+    if (n >= v.max_samples) mode = kDone;
+  }
+};
+
+// The outputs of a miss.
+ND_DEV_INLINE void write_miss(const DevView& v, const nd_gbuffer& g, int64_t r, uint32_t evals) {
+  RayResult o;
+  o.hit = false;
+  o.t = 0.0;
+  o.steps = uint32_t(v.max_steps);
+  o.evals = evals;
+  o.nx = o.ny = o.nz = 0.0f;
+  o.shadow = 1.0f;
+  o.shade = 0.0f;
+  write_result(g, nullptr, r, o);
+}
+
 }  // namespace nd
 
 namespace nd {
+
+// The hit of a listed ray: the bisection between the last sample above eps and the first
+// below it, as Lane::advance runs it inline.  *t: the hit distance, *used: the samples it
+// took.  False when march_to's loop runs out of samples first (max_steps 0): a miss.
+//
+// A bisection that runs its whole budget (exact_hit) soon halves a bracket that spans
+// one or two FP32 positions: a sample at a position whose DE one of the bracket's ends
+// has is taken from there (it counts as a sample like any other).
+template <class Set, class T, bool kDir64, bool kScenes = false>
+ND_DEV_INLINE bool resolve_hit(const DevView& v, const Dir<kDir64>& dir, const HitEntry& h, const DevScene* scenes,
+                               double* t, int* used) {
+  double a = h.a, b = h.b;
+  *used = 0;
+  *t = b;
+  if (v.verify != 0 || !(v.refine > 0 && (v.exact_hit ? b > a : b - a > march_eps<T>(v, b)))) return true;
+  int n = h.steps + 1;
+  if (n >= v.max_samples) return false;
+  const D3 o = d3(v.org[0], v.org[1], v.org[2]), d = dir.get();
+  ndw::v3<T> pa = to_t<T>(fmadd(o, d, a)), pb = to_t<T>(fmadd(o, d, b));
+  T da = T(0), db = T(0);
+  bool known_a = false, known_b = false;
+  while (true) {
+    const double st = 0.5 * (a + b);
+    const ndw::v3<T> p = to_t<T>(fmadd(o, d, st));
+    T de;
+    if (std::is_same<T, float>::value && known_a && p.x == pa.x && p.y == pa.y && p.z == pa.z) de = da;
+    else if (std::is_same<T, float>::value && known_b && p.x == pb.x && p.y == pb.y && p.z == pb.z) de = db;
+    else de = view_de<Set, T, false, kScenes>(v, p, scenes).d;
+    ++n;
+    ++*used;
+    if (below_eps<T>(de, double(de), v, st)) {
+      b = st;
+      pb = p;
+      db = de;
+      known_b = true;
+    } else {
+      a = st;
+      pa = p;
+      da = de;
+      known_a = true;
+    }
+    if ((b - a <= march_eps<T>(v, st) && !v.exact_hit) || *used >= v.refine) break;
+    if (n >= v.max_samples) return false;
+  }
+  *t = b;
+  return true;
+}
 
 // The orbit trap and changed-iteration count at a ray's hit point: the formula
 // wrapper with its trap (formula_N) evaluated once at org + dir * t_hit.

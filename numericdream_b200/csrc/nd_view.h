@@ -44,6 +44,8 @@ inline DevView make_dev_view(const nd_view_desc& v, int64_t ray_offset, int64_t 
   d.factor = std::min(std::max(v.step_safety, 0.001f), 1.0f);
   d.width = v.width;
   d.height = v.height;
+  d.inv_width = 1.0 / double(v.width);
+  d.inv_height = 1.0 / double(v.height);
   d.tile_x = v.tile_x;
   d.tile_y = v.tile_y;
   d.tile_w = v.tile_w;

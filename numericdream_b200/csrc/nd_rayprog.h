@@ -46,6 +46,7 @@ ND_DEV_INLINE double rn_add(double a, double b) { return __dadd_rn(a, b); }
 ND_DEV_INLINE double fma_d(double a, double b, double c) { return __fma_rn(a, b, c); }
 ND_DEV_INLINE float load_ro(const float* p) { return __ldg(p); }
 ND_DEV_INLINE int32_t float_bits(float x) { return __float_as_int(x); }
+ND_DEV_INLINE int32_t floor_int(float x) { return __float2int_rd(x); }  // saturates; NaN -> 0
 ND_DEV_INLINE uint32_t low_word(double x) { return uint32_t(__double2loint(x)); }
 ND_DEV_INLINE uint16_t half_bits(float x) { return __half_as_ushort(__float2half_rn(x)); }
 #else
@@ -60,6 +61,12 @@ ND_DEV_INLINE int32_t float_bits(float x) {
   int32_t b;
   memcpy(&b, &x, sizeof(b));
   return b;
+}
+ND_DEV_INLINE int32_t floor_int(float x) {
+  if (x != x) return 0;
+  if (x >= 2147483648.0f) return 2147483647;
+  if (x < -2147483648.0f) return -2147483647 - 1;
+  return int32_t(floorf(x));
 }
 ND_DEV_INLINE uint32_t low_word(double x) {
   uint64_t b;
@@ -129,7 +136,7 @@ struct DevView {
   float accel_prm[kAccelMaxCascades][4];
   float accel_inv[kAccelMaxCascades];  // 1 / cell size
   float accel_cam[3];   // the camera position the cascades are centred on (f32)
-  float accel_k;        // 1 / ((res / 2 - 1) * finest cell): lookup start level
+  float accel_k;        // 1 / ((res / 2 + 1) * finest cell), less a margin: lookup start level
   ndw::ImageRef image;  // the formula image (texels nullptr: none)
   double inv_width, inv_height;  // 1 / width, 1 / height (div_known)
   // n / d for 0 <= n < 2^31 as (n * m) >> s (DivMagic): d = the tile's pixels, d = its width
@@ -638,33 +645,43 @@ template <class T> ND_DEV_INLINE bool below_eps(const T& d, double dd, const Dev
   else return dd < march_eps<T>(v, t);
 }
 
+// skip > eps(t) for an f32 skip, likewise in f32 for the FP32 DE.
+template <class T> ND_DEV_INLINE bool above_eps(float skip, const DevView& v, double t) {
+  if constexpr (std::is_same<T, float>::value) return skip > rn_add(rn_mul(v.eps_coef, float(t)), v.eps_floor);
+  else return double(skip) > march_eps<T>(v, t);
+}
+
 // accel_skip (tpl:428-447): the safe skip recorded for the finest cascade cell that
 // holds p, 0 outside every cascade.  The cascades are nested around the camera, so
 // "finest cascade holding p" is found from p's Chebyshev distance m to the camera
 // instead of by trying every cascade: cascade l surely holds p when
-// m <= (res/2 - 1) cell_l and surely does not when m >= (res/2 + 1) cell_l, which
-// leaves cascades ceil(log2(m * accel_k)) - 1 and the one above (one more below for
-// the rounding of m * accel_k).  The cell index multiplies by 1 / cell where the
-// reference divides: the two differ only within an ulp of a cell boundary, where
-// both neighbouring cells' skips are safe to that ulp.
+// m <= (res/2 - 1) cell_l and surely does not when m >= (res/2 + 1) cell_l.  The search
+// starts at the first cascade that may hold p (accel_k is 1 / ((res/2 + 1) cell_0), less
+// a margin for the roundings), which at 64 cells a side does hold it nineteen times in
+// twenty; otherwise the next one does.  (Starting a cascade or two below, as the bound
+// (res/2 - 1) cell_l alone would have it, with six float comparisons a cascade, the lookups
+// were most of the march's instructions: 960 x 540 rays on a 64^3 x 6 grid 650 -> 471 us.)  The cell index multiplies by 1 / cell where the
+// reference divides: the two differ only within an ulp of a cell boundary, where both
+// neighbouring cells' skips are safe to that ulp.  The index is converted rounding down,
+// and an index outside [0, res) fails an unsigned comparison (the conversion saturates).
 ND_DEV_INLINE float accel_skip(const DevView& v, float px, float py, float pz) {
-  const float m = fmaxf(fabsf(px - v.accel_cam[0]), fmaxf(fabsf(py - v.accel_cam[1]), fabsf(pz - v.accel_cam[2])));
+  const float dx = px - v.accel_cam[0], dy = py - v.accel_cam[1], dz = pz - v.accel_cam[2];
+  const float m = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)));
   const float x = m * v.accel_k;
   int l = 0;
   if (x > 1.0f) {
     const int32_t b = float_bits(x);  // x > 1: a normal number (or +inf)
-    const int e = ((b >> 23) & 0xff) - 127 + ((b & 0x7fffff) != 0 ? 1 : 0);  // ceil(log2 x)
-    l = e > 2 ? e - 2 : 0;
+    l = ((b >> 23) & 0xff) - 127 + ((b & 0x7fffff) != 0 ? 1 : 0);  // ceil(log2 x)
   }
-  const float rf = float(v.accel_res);
+  const uint32_t r = uint32_t(v.accel_res);
   for (; l < v.accel_levels; ++l) {
     const float inv = v.accel_inv[l];
-    const float fx = floorf((px - v.accel_prm[l][0]) * inv);
-    const float fy = floorf((py - v.accel_prm[l][1]) * inv);
-    const float fz = floorf((pz - v.accel_prm[l][2]) * inv);
-    if (!(fx >= 0.0f && fy >= 0.0f && fz >= 0.0f && fx < rf && fy < rf && fz < rf)) continue;
-    const int r = v.accel_res;
-    return load_ro(v.accel_grid + ((int64_t(l) * r + int(fz)) * r + int(fy)) * r + int(fx));
+    const uint32_t ix = uint32_t(floor_int((px - v.accel_prm[l][0]) * inv));
+    const uint32_t iy = uint32_t(floor_int((py - v.accel_prm[l][1]) * inv));
+    const uint32_t iz = uint32_t(floor_int((pz - v.accel_prm[l][2]) * inv));
+    if (!(ix < r && iy < r && iz < r)) continue;
+    if (dx + dy + dz != dx + dy + dz) return 0.0f;  // a NaN converts to 0, which no cell holds
+    return load_ro(v.accel_grid + (((uint32_t(l) * r + iz) * r + iy) * r + ix));  // < 8 * 160^3
   }
   return 0.0f;
 }
@@ -1144,11 +1161,11 @@ template <class T, bool kDir64> struct MarchLane {
   ND_DEV_INLINE bool accel_skips(const DevView& v, int chain) {
     for (int jumps = 0;; ++jumps) {
       const D3 p = sample_pos(v);
-      const double skip = double(accel_skip(v, float(p.x), float(p.y), float(p.z)));
-      if (!(skip > march_eps<T>(v, st))) return true;
+      const float skip = accel_skip(v, float(p.x), float(p.y), float(p.z));
+      if (!above_eps<T>(skip, v, st)) return true;
       if (chain > 0 && jumps >= chain) return false;
       a = st;
-      st = st + skip;
+      st = st + double(skip);
       ++i;
       ++n;
       ++jumped;

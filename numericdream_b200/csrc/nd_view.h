@@ -114,7 +114,13 @@ inline void place_accel(DevView& d, const nd_view_desc& v, float* grid) {
     d.accel_inv[l] = 1.0f / cell;
   }
   for (int a = 0; a < 3; ++a) d.accel_cam[a] = float(v.cam_pos[a]);
-  d.accel_k = 1.0f / ((0.5f * res_f - 1.0f) * d.accel_prm[0][3]);
+  // the largest distance from the camera that the finest cascade holds: a cell past its
+  // half side, and the f32 roundings of the corner, the distance and the product (a few
+  // units of 2^-24 of the coordinates; relative to their side less for coarser cascades)
+  float cam = 0.0f;
+  for (int a = 0; a < 3; ++a) cam = std::max(cam, std::fabs(d.accel_cam[a]));
+  const float reach = (0.5f * res_f + 1.0f) * d.accel_prm[0][3];
+  d.accel_k = 1.0f / (reach + 1e-6f * (cam + reach));
 }
 
 // One scene instance as the kernels read it.  code / mcode: the instance's and its

@@ -44,23 +44,13 @@ __device__ __forceinline__ void flush_stats(Stats* s, unsigned long long rays, u
 }
 
 // Residency the kernels are compiled for: 7 blocks of 128 threads per SM with an
-// FP32 DE (at most 72 registers per thread; measured 4 % faster than 8 x 64 on the
-// batched benchmark, where 64 registers spill the ray state), 4 with an FP64 DE.
+// FP32 DE (at most 72 registers per thread), 4 with an FP64 DE.  The batched march fits
+// 64 registers, but the compiler then serialises chains it runs side by side with 70: at
+// 7 / 8 blocks 64 Mandelbulb views march in 2.43 / 2.48 ms, seven small ones (bound by
+// their longest ray's chain) in 244 / 293 us, the mixed 64-view batch in 5.27 / 5.28 ms; 6
+// blocks give 2.46 ms and 249 us.
 template <class T> struct MinBlocks {
   static constexpr int value = sizeof(T) == 4 ? 7 : 4;
-};
-// The batched FP32 march that defers its shading (the forward calls) carries no
-// normal or shadow state and fits in fewer registers.
-#ifndef ND_MARCH_MIN_BLOCKS_F32
-#define ND_MARCH_MIN_BLOCKS_F32 8
-#endif
-#ifndef ND_MARCH_MIN_BLOCKS_F64
-#define ND_MARCH_MIN_BLOCKS_F64 4
-#endif
-template <class T, bool kBatched, bool kDefer> struct MarchBlocks {
-  static constexpr int value = (sizeof(T) == 4 && kBatched && kDefer) ? ND_MARCH_MIN_BLOCKS_F32
-                               : (sizeof(T) == 8 && kDefer)            ? ND_MARCH_MIN_BLOCKS_F64
-                                                                       : MinBlocks<T>::value;
 };
 
 // --------------------------------------------------------------- plain kernel
@@ -116,7 +106,7 @@ __global__ void __launch_bounds__(128, MinBlocks<T>::value) plain_kernel(const _
 // scratch) the normal and shadow phases run inside the march.
 template <class Set, class T, bool kDir64, bool kBatched, bool kScenes = false, bool kAccel = false,
           int kBlock = 128, bool kDefer = true>
-__global__ void __launch_bounds__(kBlock, MarchBlocks<T, kBatched, kDefer>::value * 128 / kBlock)
+__global__ void __launch_bounds__(kBlock, MinBlocks<T>::value * 128 / kBlock)
     persistent_kernel(const __grid_constant__ LaunchArgs a, const __grid_constant__ DevView single) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;

@@ -335,13 +335,15 @@ template <class T> struct ParamRef {
 //
 // PR is the parameter accessor (p[i]); the adjoint instantiates the formula code
 // with dual numbers for T and a PR whose entries carry tangents.
+template <class F, class T, class PR> ND_DEV_INLINE int formula_iterations(const PR& p) {
+  const int n = F::template iterations<T, PR>(p);
+  return n < kMaxIterations ? n : kMaxIterations;
+}
 template <class F, class T, bool kTrap, class PR>
-ND_DEV_INLINE DEOut<T> formula_de_p(ndw::v3<T> pos, const PR& p, const nd_trap_desc& trap, float factor) {
+ND_DEV_INLINE DEOut<T> formula_de_p(ndw::v3<T> pos, const PR& p, const nd_trap_desc& trap, float factor, int n) {
   ndw::IterCarry<T> c{pos, T(1)};
   TrapAcc<T> acc;
   if constexpr (kTrap) acc = trap_begin<T>(trap);
-  int n = F::template iterations<T, PR>(p);
-  n = n < kMaxIterations ? n : kMaxIterations;
   int changed = 0;
   for (int it = 0; it < n; ++it) {
     if constexpr (kTrap) {
@@ -375,7 +377,8 @@ ND_DEV_INLINE DEOut<T> formula_de_p(ndw::v3<T> pos, const PR& p, const nd_trap_d
 template <class F, class T, bool kTrap>
 ND_DEV_INLINE DEOut<T> formula_de(ndw::v3<T> pos, const float* params, const nd_trap_desc& trap, float factor,
                                   const ndw::ImageRef* image = nullptr) {
-  return formula_de_p<F, T, kTrap, ParamRef<T>>(pos, ParamRef<T>{params, image}, trap, factor);
+  const ParamRef<T> p{params, image};
+  return formula_de_p<F, T, kTrap, ParamRef<T>>(pos, p, trap, factor, formula_iterations<F, T>(p));
 }
 
 // A compile-time list of formulas; code selects one (warp-uniform in practice,
@@ -392,7 +395,15 @@ template <class F> struct FormulaSet<F> {
   }
   template <class T, class PR>
   static ND_DEV_INLINE DEOut<T> de_with(int, ndw::v3<T> pos, const PR& p, const DevView& v) {
-    return formula_de_p<F, T, false, PR>(pos, p, v.trap, v.factor);
+    return formula_de_p<F, T, false, PR>(pos, p, v.trap, v.factor, formula_iterations<F, T>(p));
+  }
+  // The iteration count of a view's DE, and its distance with that count in hand (the
+  // march asks for it once a ray).
+  template <class T> static ND_DEV_INLINE int iterations(int, const DevView& v) {
+    return formula_iterations<F, T>(ParamRef<T>{v.params, &v.image});
+  }
+  template <class T> static ND_DEV_INLINE T distance(int, ndw::v3<T> pos, const DevView& v, int n) {
+    return formula_de_p<F, T, false, ParamRef<T>>(pos, ParamRef<T>{v.params, &v.image}, v.trap, v.factor, n).d;
   }
   template <class T, bool kTrap>
   static ND_DEV_INLINE DEOut<T> eval(int code, ndw::v3<T> pos, const float* params, const nd_trap_desc& trap) {
@@ -417,8 +428,17 @@ template <class F, class G, class... Rest> struct FormulaSet<F, G, Rest...> {
   }
   template <class T, class PR>
   static ND_DEV_INLINE DEOut<T> de_with(int code, ndw::v3<T> pos, const PR& p, const DevView& v) {
-    if (code == 0) return formula_de_p<F, T, false, PR>(pos, p, v.trap, v.factor);
+    if (code == 0) return formula_de_p<F, T, false, PR>(pos, p, v.trap, v.factor, formula_iterations<F, T>(p));
     return FormulaSet<G, Rest...>::template de_with<T, PR>(code - 1, pos, p, v);
+  }
+  template <class T> static ND_DEV_INLINE int iterations(int code, const DevView& v) {
+    if (code == 0) return formula_iterations<F, T>(ParamRef<T>{v.params, &v.image});
+    return FormulaSet<G, Rest...>::template iterations<T>(code - 1, v);
+  }
+  template <class T> static ND_DEV_INLINE T distance(int code, ndw::v3<T> pos, const DevView& v, int n) {
+    if (code == 0)
+      return formula_de_p<F, T, false, ParamRef<T>>(pos, ParamRef<T>{v.params, &v.image}, v.trap, v.factor, n).d;
+    return FormulaSet<G, Rest...>::template distance<T>(code - 1, pos, v, n);
   }
   template <class T, bool kTrap>
   static ND_DEV_INLINE DEOut<T> eval(int code, ndw::v3<T> pos, const float* params, const nd_trap_desc& trap) {
@@ -1130,6 +1150,7 @@ template <class T, bool kDir64> struct MarchLane {
   Dir<kDir64> dir;
   double st, a, b;
   int32_t i, k, n;
+  int32_t iters;    // the view's formula iterations (set where the kernel wants them in hand)
   uint32_t jumped;  // accelerator jumps (samples without an evaluation)
   bool hit;
 
@@ -1176,15 +1197,20 @@ template <class T, bool kDir64> struct MarchLane {
     }
   }
 
-  // Consume one DE result.
-  ND_DEV_INLINE void advance(const DevView& v, T de) {
-    const double d = double(de);
+  // Consume one DE result.  kViewInMemory: v is read from memory, not from kernel parameters.
+  template <bool kViewInMemory> ND_DEV_INLINE void advance(const DevView& v, T de) {
+    const double d = double(de), max_dist = v.max_dist;
+    const int32_t max_steps = v.max_steps;
+#if defined(__CUDA_ARCH__)
+    // read the limits here, beside the epsilon, not behind the branch
+    if constexpr (kViewInMemory) asm volatile("" ::"d"(max_dist), "r"(max_steps));
+#endif
     const bool below = below_eps<T>(de, d, v, st);
     if (mode == kProbe && !below) {
       a = st;
       st = st + d;
       ++i;
-      if (st > v.max_dist || i >= v.max_steps) mode = kDone;
+      if (st > max_dist || i >= max_steps) mode = kDone;
       return;
     }
     if (mode >= kVerify) {

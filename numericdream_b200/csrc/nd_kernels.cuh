@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::value * 128 / kBlock)
       if constexpr (kDefer) {
         const uint32_t evals = L.evals(v);
         ev_m += evals;
-        if (L.hit) hit = HitEntry{L.item, L.i, evals, 0, L.a, L.st};
+        if (L.hit) hit = HitEntry{L.item, L.i, evals, L.view, L.a, L.st};
         else write_miss(v, a.out, v.out_offset + (int64_t(L.item) - v.ray_offset), evals);
       } else {
         L.flush(v, a.out, a.t_hit);
@@ -254,11 +254,11 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::value * 128 / kBlock)
 // (the plain kernel) the pass computes the orbit trap of every ray that hit.  It
 // strides over its work with a resident grid, warp by warp (the queue appends are
 // warp-aggregated).
-#ifndef ND_SHADE_MIN_BLOCKS_F32
-#define ND_SHADE_MIN_BLOCKS_F32 7
-#endif
+// Compiled for 5 blocks per SM with an FP32 DE (no spills): at 4 / 5 / 6 / 7 blocks a
+// batch of 64 views takes 599 / 597 / 605 / 605 us, four views of 40 exact bisections 456
+// / 465 / 494 / 509 us.
 template <class T> struct ShadeBlocks {
-  static constexpr int value = sizeof(T) == 4 ? ND_SHADE_MIN_BLOCKS_F32 : MinBlocks<T>::value;
+  static constexpr int value = sizeof(T) == 4 ? 5 : MinBlocks<T>::value;
 };
 template <class Set, class T, bool kDir64, bool kBatched, bool kScenes = false, bool kAccel = false>
 __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
       HitEntry h{int32_t(i), 0, 0u, 0, 0.0, 0.0};
       if (list) h = a.hit_list[i];
       const int64_t it = h.item;
-      const int vi = kBatched ? find_view(a.views, a.nviews, it) : 0;
+      const int vi = !kBatched ? 0 : (list ? h.view : find_view(a.views, a.nviews, it));
       const DevView& v = kBatched ? a.views[vi] : single;
       const int64_t local = it - v.ray_offset;
       const int64_t r = v.out_offset + local;

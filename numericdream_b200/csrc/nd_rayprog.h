@@ -190,15 +190,15 @@ struct Stats {
   unsigned int timeouts, pad;
 };
 
-// One entry of the deferred march's hit list: the launch-local ray index, the probe steps
-// and DE evaluations its march used, and the bracket of the hit: the distance of the last
+// One entry of the deferred march's hit list: the launch-local ray index and its view, the
+// probe steps and DE evaluations its march used, and the bracket of the hit: the distance of the last
 // sample above eps and of the first below it (both the hit itself when nothing is left
 // to bisect).  The surface pass reads its hits in list order, 32 B each and coalesced.
 struct HitEntry {
   int32_t item;
   int32_t steps;
   uint32_t evals;
-  int32_t pad;
+  int32_t view;
   double a, b;
 };
 
@@ -810,7 +810,7 @@ ND_DEV_INLINE float lambert(const DevView& v, D3 dir, double nx, double ny, doub
     kx = rn_add(rn_add(-dir.x, rn_mul(v.uup[0], 0.45)), -rn_mul(v.uright[0], 0.35));
     ky = rn_add(rn_add(-dir.y, rn_mul(v.uup[1], 0.45)), -rn_mul(v.uright[1], 0.35));
     kz = rn_add(rn_add(-dir.z, rn_mul(v.uup[2], 0.45)), -rn_mul(v.uright[2], 0.35));
-    const double inv = 1.0 / sqrt(rn_add(rn_add(rn_mul(kx, kx), rn_mul(ky, ky)), rn_mul(kz, kz)));
+    const double inv = inv_sqrt(rn_add(rn_add(rn_mul(kx, kx), rn_mul(ky, ky)), rn_mul(kz, kz)));
     kx *= inv; ky *= inv; kz *= inv;
   }
   // explicitly rounded (no FMA contraction), so that every kernel gives the same bits

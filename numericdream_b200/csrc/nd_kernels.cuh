@@ -361,58 +361,68 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
 // arithmetic is shadow_visibility's, step for step, so the inline and the queued
 // pass give the same bits.  At the end of a ray: the visibility, the Lambert level
 // and the ray's evaluation count.
-template <class Set, class T, bool kScenes = false>
-__global__ void __launch_bounds__(128, MinBlocks<T>::value) shadow_kernel(const __grid_constant__ LaunchArgs a) {
+template <class Set, class T, bool kBatched, bool kScenes>
+__global__ void __launch_bounds__(128, MinBlocks<T>::value)
+    shadow_kernel(const __grid_constant__ LaunchArgs a, const __grid_constant__ DevView single) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
   const int32_t total = int32_t(*a.shadow_count);
   WarpRuns runs;
-  // this lane's shadow ray
+  // this lane's shadow ray; one that ended keeps its lane and its visibility until the
+  // next refill, when the warp writes its finished rays together
   bool busy = false;
+  float vis = 0.0f;
   int32_t qi = -1, view = 0, k = 0, sev = 0;
   double ox = 0.0, oy = 0.0, oz = 0.0, dist = 0.0, res = 1.0;
   uint32_t steps_sum = 0;
   const int64_t deadline = __shfl_sync(full, globaltimer_ns(), 0) + a.deadline_ns;
   int tick = 0;
   const int thr = a.refill_threshold;
-  auto finish = [&](float vis) {
+  constexpr bool kLoads = kBatched && !kScenes && sizeof(T) == 4;  // as in persistent_kernel
+  int iters = 0;
+  auto retire = [&]() {
+    if (busy || qi < 0) return;
     const ShadowEntry& e = a.shadow_queue[qi];
-    const DevView& v = a.views[view];
+    const DevView& v = kBatched ? a.views[view] : single;
     const int64_t r = v.out_offset + (int64_t(e.item) - v.ray_offset);
     // a view that casts shadow rays uses its light for the Lambert term (no ray direction)
     finish_at_hit(v, D3{0.0, 0.0, 0.0}, e.nx, e.ny, e.nz, vis, e.evals + uint32_t(sev), r, a.out);
     steps_sum += uint32_t(sev);
-    busy = false;
+    qi = -1;
   };
   while (true) {
-    const unsigned free_lanes = __ballot_sync(full, !busy);
-    const int nfree = __popc(free_lanes);
-    const bool have_work = runs.have_work();
-    if (!have_work && free_lanes == full) break;
-    if (have_work && nfree != 0 && (nfree >= thr || free_lanes == full)) {
-      const WarpRuns::Claim c = runs.claim(nfree, a.chunk, total, [&](int take) {
-        unsigned long long got = 0;
-        if (lane == 0) got = atomicAdd(a.shadow_counter, (unsigned long long)take);
-        return uint64_t(__shfl_sync(full, got, 0));
-      });
-      if (!busy) {
-        const int rk = __popc(free_lanes & lt_mask);
-        if (rk < c.used) {
-          qi = c.item(rk);
-          const ShadowEntry& e = a.shadow_queue[qi];
-          view = find_view_from(a.views, a.nviews, e.item, view);
-          ox = e.ox;
-          oy = e.oy;
-          oz = e.oz;
-          dist = kShadowBias;
-          res = 1.0;
-          k = 0;
-          sev = 0;
-          busy = true;
+    if (runs.have_work()) {
+      const unsigned free_lanes = __ballot_sync(full, !busy);
+      const int nfree = __popc(free_lanes);
+      if (nfree != 0 && (nfree >= thr || free_lanes == full)) {
+        retire();
+        const WarpRuns::Claim c = runs.claim(nfree, a.chunk, total, [&](int take) {
+          unsigned long long got = 0;
+          if (lane == 0) got = atomicAdd(a.shadow_counter, (unsigned long long)take);
+          return uint64_t(__shfl_sync(full, got, 0));
+        });
+        if (!busy) {
+          const int rk = __popc(free_lanes & lt_mask);
+          if (rk < c.used) {
+            qi = c.item(rk);
+            const ShadowEntry& e = a.shadow_queue[qi];
+            if constexpr (kBatched) view = find_view_from(a.views, a.nviews, e.item, view);
+            if constexpr (kLoads) iters = Set::template iterations<T>(a.views[view].code, a.views[view]);
+            ox = e.ox;
+            oy = e.oy;
+            oz = e.oz;
+            dist = kShadowBias;
+            res = 1.0;
+            k = 0;
+            sev = 0;
+            busy = true;
+          }
         }
+        continue;
       }
-      continue;
+    } else if (__all_sync(full, !busy)) {
+      break;
     }
     if (((++tick) & 63) == 0) {
       const int64_t now = __shfl_sync(full, globaltimer_ns(), 0);
@@ -422,22 +432,28 @@ __global__ void __launch_bounds__(128, MinBlocks<T>::value) shadow_kernel(const 
       }
     }
     if (busy) {
-      const DevView& v = a.views[view];
-      const D3 q = fmadd(d3(ox, oy, oz), d3(v.light[0], v.light[1], v.light[2]), dist);
-      const DEOut<T> de = view_de<Set, T, false, kScenes>(v, to_t<T>(q), a.scenes);
+      const DevView& v = kBatched ? a.views[view] : single;
+      const ndw::v3<T> q = to_t<T>(fmadd(d3(ox, oy, oz), d3(v.light[0], v.light[1], v.light[2]), dist));
+      double d;
+      if constexpr (kLoads) d = double(Set::template distance<T>(v.code, q, v, iters));
+      else d = double(view_de<Set, T, false, kScenes>(v, q, a.scenes).d);
       ++sev;
-      const double d = double(de.d);
       if (d < kShadowHitEps) {
-        finish(0.0f);
+        vis = 0.0f;
+        busy = false;
       } else {
         res = fmin(res, double(v.shadow_k) * d / dist);
         dist += fmax(d, kShadowMinStep);
         ++k;
         const int steps = v.max_steps < kShadowMaxSteps ? v.max_steps : kShadowMaxSteps;
-        if (k >= steps || dist >= 2.0 * v.max_dist) finish(float(fmin(fmax(res, 0.0), 1.0)));
+        if (k >= steps || dist >= 2.0 * v.max_dist) {
+          vis = float(fmin(fmax(res, 0.0), 1.0));
+          busy = false;
+        }
       }
     }
   }
+  retire();
   unsigned long long s = steps_sum;
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
   if (lane == 0 && s) {
@@ -532,10 +548,13 @@ typedef cudaError_t (*ShadeFn)(const LaunchArgs&, const DevView&, const LaunchCo
 // The shadow pass over a launch's shadow queue: a resident grid (its size cannot
 // depend on the queue length, which the surface pass writes on the device), runs of
 // up to 16 queue entries per warp claim.
-template <class Set, class T, bool kScenes = false>
-cudaError_t launch_shadow(const LaunchArgs& a, const LaunchConfig& c, cudaStream_t s) {
+template <class Set, class T, bool kScenes = false, bool kBatched = true>
+cudaError_t launch_shadow(const LaunchArgs& a, const DevView& single, const LaunchConfig& c, cudaStream_t s) {
+  // one view's constants travel in the kernel's parameters, as in the march
+  if constexpr (kBatched && !kScenes)
+    if (a.nviews == 1) return launch_shadow<Set, T, kScenes, false>(a, single, c, s);
   int per_sm = 0;
-  cudaError_t e = resident_blocks(shadow_kernel<Set, T, kScenes>, 128, c.blocks_per_sm, &per_sm);
+  cudaError_t e = resident_blocks(shadow_kernel<Set, T, kBatched, kScenes>, 128, c.blocks_per_sm, &per_sm);
   if (e != cudaSuccess) return e;
   int64_t grid = int64_t(per_sm) * c.num_sms;
   const int64_t needed = (a.total_rays + 127) / 128;  // at most one queue entry per ray
@@ -543,23 +562,24 @@ cudaError_t launch_shadow(const LaunchArgs& a, const LaunchConfig& c, cudaStream
   if (grid <= 0) return cudaSuccess;
   LaunchArgs b = a;
   b.chunk = 16;
-  shadow_kernel<Set, T, kScenes><<<unsigned(grid), 128, 0, s>>>(b);
+  shadow_kernel<Set, T, kBatched, kScenes><<<unsigned(grid), 128, 0, s>>>(b, single);
   return cudaGetLastError();
 }
 
-typedef cudaError_t (*ShadowFn)(const LaunchArgs&, const LaunchConfig&, cudaStream_t);
+typedef cudaError_t (*ShadowFn)(const LaunchArgs&, const DevView&, const LaunchConfig&, cudaStream_t);
 
 // --------------------------------------------------------------- lite shading
 // One thread per ray of the call (resident grid, strided): misses take the view's
 // background, hits lite_at_hit from the forward's depth64 / normal / trap.
-template <class Set, class T, bool kDir64, bool kScenes = false>
+template <class Set, class T, bool kDir64, bool kScenes, bool kBatched>
 __global__ void __launch_bounds__(128, MinBlocks<T>::value)
-    lite_kernel(const __grid_constant__ LaunchArgs a, const nd_lite_desc* __restrict__ lites,
+    lite_kernel(const __grid_constant__ LaunchArgs a, const __grid_constant__ DevView single,
+                const nd_lite_desc* __restrict__ lites,
                 const nd_lite_desc* __restrict__ scene_colors, float4* __restrict__ rgba) {
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.total_rays; i += stride) {
-    const int vi = find_view(a.views, a.nviews, i);
-    const DevView& v = a.views[vi];
+    const int vi = kBatched ? find_view(a.views, a.nviews, i) : 0;
+    const DevView& v = kBatched ? a.views[vi] : single;
     const nd_lite_desc& L = lites[vi];
     const int64_t local = i - v.ray_offset;
     const int64_t r = v.out_offset + local;
@@ -575,22 +595,25 @@ __global__ void __launch_bounds__(128, MinBlocks<T>::value)
   }
 }
 
-template <class Set, class T, bool kDir64, bool kScenes = false>
-cudaError_t launch_lite(const LaunchArgs& a, const nd_lite_desc* lites, const nd_lite_desc* scene_colors, float* rgba,
+template <class Set, class T, bool kDir64, bool kScenes = false, bool kBatched = true>
+cudaError_t launch_lite(const LaunchArgs& a, const DevView& single, const nd_lite_desc* lites, const nd_lite_desc* scene_colors, float* rgba,
                         int num_sms, cudaStream_t s) {
+  if constexpr (kBatched && !kScenes)
+    if (a.nviews == 1) return launch_lite<Set, T, kDir64, kScenes, false>(a, single, lites, scene_colors, rgba, num_sms, s);
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lite_kernel<Set, T, kDir64, kScenes>, 128, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, lite_kernel<Set, T, kDir64, kScenes, kBatched>, 128, 0);
   if (e != cudaSuccess) return e;
   int64_t grid = int64_t(std::max(per_sm, 1)) * num_sms;
   const int64_t needed = (a.total_rays + 127) / 128;
   if (grid > needed) grid = needed;
   if (grid <= 0) return cudaSuccess;
-  lite_kernel<Set, T, kDir64, kScenes><<<unsigned(grid), 128, 0, s>>>(a, lites, scene_colors,
-                                                                      reinterpret_cast<float4*>(rgba));
+  lite_kernel<Set, T, kDir64, kScenes, kBatched><<<unsigned(grid), 128, 0, s>>>(a, single, lites, scene_colors,
+                                                                                reinterpret_cast<float4*>(rgba));
   return cudaGetLastError();
 }
 
-typedef cudaError_t (*LiteFn)(const LaunchArgs&, const nd_lite_desc*, const nd_lite_desc*, float*, int, cudaStream_t);
+typedef cudaError_t (*LiteFn)(const LaunchArgs&, const DevView&, const nd_lite_desc*, const nd_lite_desc*, float*, int, cudaStream_t);
 
 // --------------------------------------------------------------- accelerator build
 // cs_build_accel (tpl:5412-5431): one thread per voxel of every accelerated view of

@@ -672,7 +672,7 @@ nd_status enqueue(nd_ctx* ctx, const nd_view_desc* views, int nviews, const nd_m
           if (!hf) return fail(ctx, ND_ERR_UNSUPPORTED, "no shadow kernels in this formula set");
           LaunchConfig sc2 = c;
           sc2.blocks_per_sm = 0;
-          e = hf(a, sc2, stream);
+          e = hf(a, h_views[base], sc2, stream);
           if (e != cudaSuccess) return cuda_fail(ctx, e, "shadow pass launch");
         }
       }
@@ -1654,7 +1654,7 @@ nd_status shade_lite_impl(nd_ctx* ctx, const nd_view_desc* views, int32_t nviews
       fn = L.table.scene_lite_f32;
       if (!fn) return fail(ctx, ND_ERR_UNSUPPORTED, "no scene kernels in this formula set");
     }
-    e = fn(a, ctx->d_lite + base, ctx->d_lite + nviews, rgba, ctx->num_sms, st);
+    e = fn(a, ctx->h_views[base], ctx->d_lite + base, ctx->d_lite + nviews, rgba, ctx->num_sms, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "lite shading launch");
     base += nv;
   }

@@ -55,3 +55,17 @@ def test_deferred_march_equals_the_plain_launch(ctx, form, precision):
             a, b = getattr(out[0], name), getattr(out[1], name)
             assert torch.equal(a, b), f"{name}: {(a != b).sum().item()} values differ"
         assert counts[0] == counts[1]
+
+
+def test_lite_and_shadows_of_one_view_equal_those_in_a_batch(ctx):
+    """One view's constants travel in kernel parameters, a batch's in memory: the same bits."""
+    views = [_view("central_shadow", 61, 43), _view("central_shadow", 17, 9, 2)]
+    lite = abi.make_lite([((0.1, 0.2, 0.3), 0.0, 0.4, 1.4), ((0.9, 0.5, 0.2), 1.0, 0.7, 1.6)],
+                         [(abi.ND_LIGHT_GLOBAL, (0.4, 0.8, -0.45), (1.0, 0.9, 0.8), 1.1)])
+
+    def outputs(vs):
+        g = runtime.GBuffer.allocate(workloads.rays(vs))
+        ctx.forward(vs, g, runtime.make_opts(kernel=abi.ND_KERNEL_PERSISTENT))
+        return torch.cat([ctx.shade_lite(vs, [lite] * len(vs), g), g.shadow[:, None], g.shade[:, None]], 1)
+
+    assert torch.equal(outputs(views), torch.cat([outputs([v]) for v in views]))

@@ -53,6 +53,20 @@ template <class T> struct MinBlocks {
   static constexpr int value = sizeof(T) == 4 ? 7 : 4;
 };
 
+// The n-th ray of a view in blocks of 8 x 4 pixels (a warp's 32 rays), row of blocks by row
+// of blocks: a permutation of the rays of each sample plane, whatever the tile's size.
+ND_DEV_INLINE int64_t block_order(const DevView& v, int64_t n) {
+  const int64_t npix = int64_t(v.tile_w) * v.tile_h;
+  if (npix >= 0x40000000ll || v.rays >= 0x7fffffffll) return n;
+  const uint32_t w = uint32_t(v.tile_w), sample = div_by(uint32_t(n), v.npix_m, v.npix_s);
+  const uint32_t pix = uint32_t(n) - sample * uint32_t(npix);
+  const uint32_t band = div_by(pix >> 2, v.width_m, v.width_s);  // pix / (4 w)
+  const uint32_t in = pix - band * 4 * w, rows = min(4u, uint32_t(v.tile_h) - 4 * band);
+  const uint32_t block = in / (8 * rows), at = in - block * 8 * rows, cols = min(8u, w - 8 * block);
+  const uint32_t y = at / cols, x = at - y * cols;
+  return int64_t(sample) * npix + int64_t(4 * band + y) * w + 8 * block + x;
+}
+
 // --------------------------------------------------------------- plain kernel
 // The reference's per-pixel program as a plain per-view launch: one thread per
 // ray, the march loop of march_to, then the normal taps of estimate_normal, then
@@ -61,7 +75,14 @@ template <class T> struct MinBlocks {
 template <class Set, class T, bool kDir64>
 __global__ void __launch_bounds__(128, MinBlocks<T>::value) plain_kernel(const __grid_constant__ LaunchArgs a,
                                                     const __grid_constant__ DevView v) {
-  const int64_t local = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;  // ray index inside the view
+  const int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  // The ray index inside the view.  A warp of a 8 x 4 pixel block has more of its lanes
+  // alike than one of 32 pixels in a row: an FP32 view of 256 x 256 takes 281 us against
+  // 291.  With fewer warps than would keep the schedulers busy nothing is gained (96 x 54
+  // rays: 186 against 184 us), nor with an FP64 DE; the persistent march, whose lanes
+  // drift apart as they refill, was 1 to 3 % slower with it.
+  const bool blocks = sizeof(T) == 4 && v.rays >= 16384 && thread < v.rays;
+  const int64_t local = blocks ? block_order(v, thread) : thread;
   unsigned long long rays = 0, hits = 0, m = 0, nn = 0, sh = 0;
   if (local < v.rays) {
     Lane<T, kDir64> L;

@@ -69,3 +69,21 @@ def test_lite_and_shadows_of_one_view_equal_those_in_a_batch(ctx):
         return torch.cat([ctx.shade_lite(vs, [lite] * len(vs), g), g.shadow[:, None], g.shade[:, None]], 1)
 
     assert torch.equal(outputs(views), torch.cat([outputs([v]) for v in views]))
+
+
+@pytest.mark.parametrize("w,h,spp", [(191, 97, 1), (130, 127, 1), (16391, 1, 1), (1, 16384, 1), (3, 5462, 2), (65, 127, 2),
+                                     (128, 128, 1)])
+def test_plain_launch_in_blocks_marches_every_ray(ctx, w, h, spp):
+    """Views large enough for the plain launch's 8 x 4 blocks: tiles that no block fits, and
+    remainders on both sides."""
+    v = _view("bisect4", w, h, spp)
+    n = workloads.rays([v])
+    out = []
+    for kernel in (abi.ND_KERNEL_PLAIN, abi.ND_KERNEL_PERSISTENT):
+        g = runtime.GBuffer.allocate(n)
+        g.steps.fill_(-1)
+        ctx.forward([v], g, runtime.make_opts(kernel=kernel))
+        assert ctx.stats().rays == n
+        out.append(g)
+    for name in ("depth", "normal", "trap", "steps", "evals"):
+        assert torch.equal(getattr(out[0], name), getattr(out[1], name)), name

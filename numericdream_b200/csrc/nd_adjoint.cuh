@@ -67,9 +67,9 @@ struct LitRay {
 constexpr int64_t kAdjointRays = int64_t(1) << 22;
 // Blocks of 128 threads per SM the adjoint kernels are compiled for: surface FP32 and
 // FP64, thetas FP32 and FP64.  Measured for the thetas: FP32 5 / 6 / 8 blocks 978 / 1024 /
-// 1003 us a backward of 4 views of 512 x 512; FP64 2 / 3 / 4 blocks 1021 / 856 / 879 us
-// a backward of 2 views of 256 x 256.
-constexpr int kSurfaceBlocks32 = 6, kSurfaceBlocks64 = 4, kThetaBlocks32 = 5, kThetaBlocks64 = 3;
+// 1003 us a backward of 4 views of 512 x 512; FP64 3 / 4 blocks (146 registers; 128 with 12
+// bytes spilled) 1717 / 1530 us a backward of 2 views of 256 x 256.
+constexpr int kSurfaceBlocks32 = 6, kSurfaceBlocks64 = 4, kThetaBlocks32 = 5, kThetaBlocks64 = 4;
 
 // Parameter accessor with one dual tangent: parameter `seed` gets tangent 1.
 template <class S> struct DualParams {
@@ -88,26 +88,6 @@ ND_DEV_INLINE ndw::Dual<S> de_dir_full(const DevView& v, D3 p, D3 tan, int seed)
 template <class Set, class S>
 ND_DEV_INLINE S de_dir(const DevView& v, D3 p, D3 tan, int seed) {
   return de_dir_full<Set, S>(v, p, tan, seed).d;
-}
-
-// Parameter accessor with dual tangents: parameter seed[i] has 1 in tangent i.
-template <class S, int N> struct DualsParams {
-  const float* v;
-  const int* seed;
-  ND_DEV_INLINE ndw::Duals<S, N> operator[](int i) const {
-    return ndw::mkds<N>(S(v[i]), [&](int k) { return i == seed[k] ? S(1) : S(0); });
-  }
-};
-
-// The DE of view v at p and its N derivatives along (position tangent tan[i], parameter
-// seed[i]).
-template <class Set, class S, int N>
-ND_DEV_INLINE ndw::Duals<S, N> de_dirs(const DevView& v, D3 p, const D3* tan, const int* seed) {
-  typedef ndw::Duals<S, N> DS;
-  const ndw::v3<DS> q(ndw::mkds<N>(S(p.x), [&](int i) { return S(tan[i].x); }),
-                      ndw::mkds<N>(S(p.y), [&](int i) { return S(tan[i].y); }),
-                      ndw::mkds<N>(S(p.z), [&](int i) { return S(tan[i].z); }));
-  return Set::template de_with<DS, DualsParams<S, N>>(v.code, q, DualsParams<S, N>{v.params, seed}, v).d;
 }
 
 // Largest |DE(p) - eps(t)| / eps(t) at a hit that is a root of the level set.  FP64
@@ -157,65 +137,34 @@ ND_DEV_INLINE D3 adjoint_tangent(const PoseTangents& T, const AdjointRay& r, int
   return axpy(dorg, r.t, dd);
 }
 
-// dI/dtheta_k of one ray for the C thetas from k0 on.
-template <class Set, class S, int C>
-ND_DEV_INLINE void adjoint_thetas(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
-                                  const AdjointRay& r, double denom, const D3& D, int k0, double* dI) {
-  const double Dn = sqrt(dot3(D, D));
+// dI/dtheta_k of one ray, one tangent to an evaluation.  Three FP64 tangents to an evaluation
+// would share its arccosine, powers and sines (0.83 ms where one takes 1.53), but the compiler
+// then fuses other products, in the values too, and a grazing ray turns an ulp of those into
+// 1e-9 to 1e-7 of its derivatives.
+template <class Set, class S>
+ND_DEV_INLINE double adjoint_theta(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
+                                   const AdjointRay& r, double denom, const D3& D, int k) {
+  // |D| as adjoint_surface has it: its sum is fused in this order there, left to the compiler
+  // in another one here
+  const double Dn = sqrt(fma_d(D.z, D.z, fma_d(D.x, D.x, rn_mul(D.y, D.y))));
   const D3 n = D3{D.x / Dn, D.y / Dn, D.z / Dn};
   const D3 L = D3{v.light[0], v.light[1], v.light[2]};
-  if constexpr (C == 1) {
-    const int seed = k0 < nparam ? param_idx[k0] : -1;
-    const D3 ptan0 = adjoint_tangent(T, r, k0, nparam);
-    const double a_k = double(de_dir<Set, S>(v, r.p, ptan0, seed));
-    const double dt = -a_k / denom;
-    const D3 dp = axpy(ptan0, dt, r.d);
-    const double dh = r.hc * dt;
-    double dD[3];
-    for (int i = 0; i < 3; ++i) {
-      const D3 tp = axpy(dp, dh, axis(i, 1.0));
-      const D3 tm = axpy(dp, -dh, axis(i, 1.0));
-      dD[i] = double(de_dir<Set, S>(v, axpy(r.p, r.h, axis(i, 1.0)), tp, seed)) -
-              double(de_dir<Set, S>(v, axpy(r.p, -r.h, axis(i, 1.0)), tm, seed));
-    }
-    const double nd = n.x * dD[0] + n.y * dD[1] + n.z * dD[2];
-    const D3 dn = D3{(dD[0] - n.x * nd) / Dn, (dD[1] - n.y * nd) / Dn, (dD[2] - n.z * nd) / Dn};
-    dI[0] = (1.0 - kSimpleAmbient) * dot3(L, dn);
-  } else {
-    int seed[C];
-    D3 tan[C];
-    double dt[C], sum[C];  // sum: n . dD, then L . dD
-    for (int c = 0; c < C; ++c) {
-      seed[c] = k0 + c < nparam ? param_idx[k0 + c] : -1;
-      tan[c] = adjoint_tangent(T, r, k0 + c, nparam);
-      dt[c] = 0.0;
-    }
-    double nd[C];
-    for (int c = 0; c < C; ++c) sum[c] = nd[c] = 0.0;
-    // one call site: the evaluation at the hit (tap -1), then the six taps
-#pragma unroll 1
-    for (int tap = -1; tap < 6; ++tap) {
-      const int i = tap < 0 ? 0 : tap >> 1;
-      const double s = tap < 0 ? 0.0 : (tap & 1 ? -1.0 : 1.0);
-      D3 at[C];
-      for (int c = 0; c < C; ++c) {
-        const D3 dp = axpy(tan[c], dt[c], r.d);
-        at[c] = axpy(dp, s * r.hc * dt[c], axis(i, 1.0));
-      }
-      const ndw::Duals<S, C> e = de_dirs<Set, S, C>(v, axpy(r.p, s * r.h, axis(i, 1.0)), at, seed);
-      const double ni = i == 0 ? n.x : i == 1 ? n.y : n.z, Li = i == 0 ? L.x : i == 1 ? L.y : L.z;
-      for (int c = 0; c < C; ++c) {
-        if (tap < 0) {
-          dt[c] = -double(e.d[c]) / denom;
-        } else {
-          nd[c] += s * ni * double(e.d[c]);
-          sum[c] += s * Li * double(e.d[c]);
-        }
-      }
-    }
-    // L . dn with dn = (dD - n (n . dD)) / |D|
-    for (int c = 0; c < C; ++c) dI[c] = (1.0 - kSimpleAmbient) * (sum[c] - dot3(L, n) * nd[c]) / Dn;
+  const int seed = k < nparam ? param_idx[k] : -1;
+  const D3 ptan0 = adjoint_tangent(T, r, k, nparam);
+  const double a_k = double(de_dir<Set, S>(v, r.p, ptan0, seed));
+  const double dt = -a_k / denom;
+  const D3 dp = axpy(ptan0, dt, r.d);
+  const double dh = r.hc * dt;
+  double dD[3];
+  for (int i = 0; i < 3; ++i) {
+    const D3 tp = axpy(dp, dh, axis(i, 1.0));
+    const D3 tm = axpy(dp, -dh, axis(i, 1.0));
+    dD[i] = double(de_dir<Set, S>(v, axpy(r.p, r.h, axis(i, 1.0)), tp, seed)) -
+            double(de_dir<Set, S>(v, axpy(r.p, -r.h, axis(i, 1.0)), tm, seed));
   }
+  const double nd = n.x * dD[0] + n.y * dD[1] + n.z * dD[2];
+  const D3 dn = D3{(dD[0] - n.x * nd) / Dn, (dD[1] - n.y * nd) / Dn, (dD[2] - n.z * nd) / Dn};
+  return (1.0 - kSimpleAmbient) * dot3(L, dn);
 }
 
 // What the derivatives along every theta share: g . d - coef and the normal's
@@ -223,29 +172,22 @@ ND_DEV_INLINE void adjoint_thetas(const DevView& v, const PoseTangents& T, const
 // normal, a degenerate gradient, a hit on a jump of the DE).
 //
 // The FP32 form ends in the loop over the first `thetas` derivatives, which the kernels
-// run zero times (adjoint_thetas computes them for the lit rays): the compiler contracts
-// the gradient's products into FMAs by what surrounds them, and with the loop there the
-// derivatives keep the rounding they had when one lane computed all of them.
+// run zero times (adjoint_theta computes them for the lit rays): the compiler contracts the
+// gradient's products into FMAs by what surrounds them, and with the loop there the
+// derivatives keep the rounding they had when one lane computed all of them.  Without it
+// the gradient's x component is up to 16 ulps off and the rows 1e-6 in norm (an opaque
+// seed or axis, a function of its own, another order of the axes and fused operators of the
+// duals move them as much or more); it costs 15 us of 884.  FP64 rows keep their bits
+// without it.
 template <class Set, class S>
 ND_DEV_INLINE bool adjoint_surface(const DevView& v, const PoseTangents& T, const int32_t* param_idx, int nparam,
                                    int thetas, const AdjointRay& r, double* denom, double* Dv, double* dI) {
   // value and gradient of the DE at the hit
-  D3 g;
-  double value;
-  if constexpr (sizeof(S) == 8) {
-    const D3 axes[3] = {axis(0, 1.0), axis(1, 1.0), axis(2, 1.0)};
-    const int none[3] = {-1, -1, -1};
-    const ndw::Duals<S, 3> e = de_dirs<Set, S, 3>(v, r.p, axes, none);
-    value = e.v;
-    g = D3{e.d[0], e.d[1], e.d[2]};
-  } else {
-    const ndw::Dual<S> gx = de_dir_full<Set, S>(v, r.p, axis(0, 1.0), -1);
-    g = D3{double(gx.d), double(de_dir<Set, S>(v, r.p, axis(1, 1.0), -1)),
-           double(de_dir<Set, S>(v, r.p, axis(2, 1.0), -1))};
-    value = double(gx.v);
-  }
+  const ndw::Dual<S> gx = de_dir_full<Set, S>(v, r.p, axis(0, 1.0), -1);
+  const D3 g = D3{double(gx.d), double(de_dir<Set, S>(v, r.p, axis(1, 1.0), -1)),
+                  double(de_dir<Set, S>(v, r.p, axis(2, 1.0), -1))};
   const double eps_t = double(v.eps_coef) * r.t + double(v.eps_floor);
-  if (eps_t > 0.0 && !(fabs(value - eps_t) <= RootTol<S>::value * eps_t)) return false;
+  if (eps_t > 0.0 && !(fabs(double(gx.v) - eps_t) <= RootTol<S>::value * eps_t)) return false;
   *denom = dot3(g, r.d) - double(v.eps_coef);
   // the normal's central-difference vector D
   for (int i = 0; i < 3; ++i)
@@ -257,7 +199,7 @@ ND_DEV_INLINE bool adjoint_surface(const DevView& v, const PoseTangents& T, cons
   const D3 n = D3{D.x / Dn, D.y / Dn, D.z / Dn};
   if (!(dot3(n, D3{v.light[0], v.light[1], v.light[2]}) > 0.0)) return false;
   if constexpr (sizeof(S) == 4)
-    for (int k = 0; k < thetas; ++k) adjoint_thetas<Set, S, 1>(v, T, param_idx, nparam, r, *denom, D, k, dI + k);
+    for (int k = 0; k < thetas; ++k) dI[k] = adjoint_theta<Set, S>(v, T, param_idx, nparam, r, *denom, D, k);
   return true;
 }
 
@@ -303,15 +245,12 @@ __global__ static void __launch_bounds__(256) adjoint_list_kernel(const __grid_c
 // The adjoint of a listed hit is two kernels.  The first, one lane per hit, does what all
 // thetas share: the DE's value and gradient at the hit and its values at the six normal
 // taps.  About half of the hits end there (back-lit normals).  The second does a lit ray's
-// K = nparam + 3 derivatives, 7 dual evaluations each, C thetas to an evaluation: C = 1
-// for FP32 duals, whose tangents cost as much as their values, 3 for FP64 duals, whose
-// values (64-bit arccosine, powers, sines) are most of an evaluation.  Both lists are
-// dense, so that no lane waits for a neighbour that missed, was back-lit or had no weight:
-// one kernel with one lane per ray of the image and one tangent per evaluation ran with 15
-// (FP32) and 13 (FP64) of 32 lanes active.  The kernels are bound by instruction issue
-// (FP32) and by the FP64 pipe's latency (FP64, 168 registers).  A backward call with two
-// parameters: 4 views of 512 x 512, FP32, 2.10 -> 1.00 ms; 2 views of 256 x 256, FP64,
-// 4.07 -> 0.83 ms.
+// K = nparam + 3 derivatives, 7 dual evaluations each.  Both lists are dense, so that no
+// lane waits for a neighbour that missed, was back-lit or had no weight: one kernel with one
+// lane per ray of the image ran with 15 (FP32) and 13 (FP64) of 32 lanes active.  The
+// kernels are bound by instruction issue (FP32) and by the FP64 pipe's latency (FP64).  A
+// backward call with two parameters: 4 views of 512 x 512, FP32, 2.19 -> 0.89 ms; 2 views of
+// 256 x 256, FP64, 4.12 -> 1.53 ms.
 template <class Set, class S>
 __global__ void __launch_bounds__(128, sizeof(S) == 4 ? kSurfaceBlocks32 : kSurfaceBlocks64)
     adjoint_surface_kernel(const __grid_constant__ AdjointArgs a) {
@@ -337,38 +276,32 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4 ? kSurfaceBlocks32 : kSurf
   }
 }
 
-// One lane per lit ray and chunk of C thetas; the chunks of a ray are
-// neighbours.  A lane keeps its chunk from one ray to the next (the stride is a multiple
-// of the chunks), so it sums its view's gradient in registers.
-template <class Set, class S, int C>
+// One lane per lit ray and theta; the thetas of a ray are neighbours.  A lane keeps its
+// theta from one ray to the next (the stride is a multiple of the thetas), so it sums its
+// view's gradient in a register.
+template <class Set, class S>
 __global__ void __launch_bounds__(128, sizeof(S) == 4 ? kThetaBlocks32 : kThetaBlocks64)
     adjoint_theta_kernel(const __grid_constant__ AdjointArgs a) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int K = a.nparam + kPoseParams;
-  const int chunks = (K + C - 1) / C;
-  const int64_t items = int64_t(a.counts[1]) * chunks;
-  const int64_t threads = int64_t(gridDim.x) * blockDim.x;
-  const int64_t stride = threads / chunks * chunks;
+  const int64_t items = int64_t(a.counts[1]) * K;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x / K * K;
   const int64_t me = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int k0 = int(me % chunks) * C;
-  double acc[C];
-  for (int c = 0; c < C; ++c) acc[c] = 0.0;
+  const int mine = int(me % K);
+  double acc = 0.0;
   int cur = -1;
   // adds the sums of the lanes whose view is not `keep`: one atomic per view and theta
   auto flush = [&](int keep) {
     unsigned left = __ballot_sync(full, cur >= 0 && cur != keep);
     while (left) {
       const int src = __ffs(left) - 1;
-      const int view = __shfl_sync(full, cur, src), k = __shfl_sync(full, k0, src);
-      const bool in = cur == view && k0 == k && cur != keep;
+      const int view = __shfl_sync(full, cur, src), k = __shfl_sync(full, mine, src);
+      const bool in = cur == view && mine == k && cur != keep;
       left &= ~__ballot_sync(full, in);
-      for (int c = 0; c < C; ++c) {
-        if (k + c >= K) break;
-        double x = in ? acc[c] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(full, x, o);
-        if (lane == 0 && x != 0.0) atomicAdd(&a.grad[int64_t(a.views[view].user_index) * K + k + c], x);
-      }
+      double x = in ? acc : 0.0;
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(full, x, o);
+      if (lane == 0 && x != 0.0) atomicAdd(&a.grad[int64_t(a.views[view].user_index) * K + k], x);
       if (in) cur = -1;
     }
   };
@@ -376,28 +309,24 @@ __global__ void __launch_bounds__(128, sizeof(S) == 4 ? kThetaBlocks32 : kThetaB
     const int64_t item = base + lane;
     const bool live = item < items && me < stride;
     LitRay o;
-    if (live) o = a.lit[item / chunks];
+    if (live) o = a.lit[item / K];
     if (a.grad) {
       const int view = live ? o.view : cur;
       if (__any_sync(full, cur >= 0 && view != cur)) flush(view);
       if (live && cur < 0) {
         cur = view;
-        for (int c = 0; c < C; ++c) acc[c] = 0.0;
+        acc = 0.0;
       }
     }
     if (live) {
       const DevView& v = a.views[o.view];
       const int64_t local = a.first + o.ray - v.ray_offset;
       const int64_t r = v.out_offset + local;
-      double dI[C];
-      adjoint_thetas<Set, S, C>(v, a.tangents[o.view], a.param_idx, a.nparam, adjoint_ray(v, local, a.depth64[r]),
-                                o.denom, D3{o.D[0], o.D[1], o.D[2]}, k0, dI);
-      const double w = a.grad ? double(a.dL_dshade[r]) : 0.0;
-      for (int c = 0; c < C; ++c) {
-        if (k0 + c >= K) break;
-        if (a.dshade) a.dshade[r * K + k0 + c] = dI[c];
-        acc[c] += w * dI[c];
-      }
+      const double dI = adjoint_theta<Set, S>(v, a.tangents[o.view], a.param_idx, a.nparam,
+                                              adjoint_ray(v, local, a.depth64[r]), o.denom,
+                                              D3{o.D[0], o.D[1], o.D[2]}, mine);
+      if (a.dshade) a.dshade[r * K + mine] = dI;
+      acc += (a.grad ? double(a.dL_dshade[r]) : 0.0) * dI;
     }
   }
   if (a.grad) flush(-2);
@@ -414,8 +343,6 @@ template <class Kernel> cudaError_t launch_listed(Kernel kernel, const AdjointAr
 }
 
 template <class Set, class S> cudaError_t launch_adjoint(AdjointArgs a, cudaStream_t s) {
-  constexpr int C = sizeof(S) == 4 ? 1 : 3;
-  const int chunks = (a.nparam + kPoseParams + C - 1) / C;
   for (a.first = 0; a.first < a.total_rays; a.first = a.last) {
     a.last = a.total_rays - a.first > kAdjointRays ? a.first + kAdjointRays : a.total_rays;
     const int64_t n = a.last - a.first;
@@ -424,7 +351,7 @@ template <class Set, class S> cudaError_t launch_adjoint(AdjointArgs a, cudaStre
     adjoint_list_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(a);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = launch_listed(adjoint_surface_kernel<Set, S>, a, n, s);
-    if (e == cudaSuccess) e = launch_listed(adjoint_theta_kernel<Set, S, C>, a, n * chunks, s);
+    if (e == cudaSuccess) e = launch_listed(adjoint_theta_kernel<Set, S>, a, n * (a.nparam + kPoseParams), s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

@@ -124,155 +124,4 @@ template <class S> ND_HD_INLINE void sin_cos(Dual<S> x, Dual<S>& s, Dual<S>& c) 
   c = mkd(cv, -sv * x.d);
 }
 
-template <class S, int N> struct Duals {
-  S v;
-  S d[N];
-  ND_HD_INLINE Duals() : Duals(S(0), 0) {}
-  ND_HD_INLINE Duals(float x) : Duals(S(x), 0) {}
-  ND_HD_INLINE Duals(double x) : Duals(S(x), 0) {}
-  ND_HD_INLINE Duals(int x) : Duals(S(x), 0) {}
-  ND_HD_INLINE Duals(unsigned x) : Duals(S(x), 0) {}
-  ND_HD_INLINE Duals(S x, int) : v(x) {
-    for (int i = 0; i < N; ++i) d[i] = S(0);
-  }
-  ND_HD_INLINE explicit operator float() const { return float(v); }
-  ND_HD_INLINE explicit operator double() const { return double(v); }
-  ND_HD_INLINE Duals& operator+=(Duals o) { return *this = *this + o; }
-  ND_HD_INLINE Duals& operator-=(Duals o) { return *this = *this - o; }
-  ND_HD_INLINE Duals& operator*=(Duals o) { return *this = *this * o; }
-  ND_HD_INLINE Duals& operator/=(Duals o) { return *this = *this / o; }
-};
-
-// A dual with value v and the tangents f(0), ..., f(N - 1).
-template <int N, class S, class F> ND_HD_INLINE Duals<S, N> mkds(S v, F f) {
-  Duals<S, N> r(v, 0);
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = f(i);
-  return r;
-}
-// Divides tangents by x.
-template <class S> struct Divisor {
-  S x;
-  ND_HD_INLINE explicit Divisor(S a) : x(std::is_same<S, double>::value ? S(1) / a : a) {}
-  ND_HD_INLINE S operator()(S a) const { return std::is_same<S, double>::value ? a * x : a / x; }
-};
-
-#define ND_DUAL template <class S, int N> ND_HD_INLINE
-#define ND_DUAL1 ND_DUAL Duals<S, N>
-ND_DUAL1 operator+(Duals<S, N> a, Duals<S, N> b) {
-  return mkds<N>(a.v + b.v, [&](int i) { return a.d[i] + b.d[i]; });
-}
-ND_DUAL1 operator-(Duals<S, N> a, Duals<S, N> b) {
-  return mkds<N>(a.v - b.v, [&](int i) { return a.d[i] - b.d[i]; });
-}
-ND_DUAL1 operator*(Duals<S, N> a, Duals<S, N> b) {
-  return mkds<N>(a.v * b.v, [&](int i) { return a.d[i] * b.v + a.v * b.d[i]; });
-}
-ND_DUAL1 operator/(Duals<S, N> a, Duals<S, N> b) {
-  const S q = a.v / b.v;
-  const Divisor<S> by(b.v);
-  return mkds<N>(q, [&](int i) { return by(a.d[i] - q * b.d[i]); });
-}
-ND_DUAL1 operator-(Duals<S, N> a) {
-  return mkds<N>(-a.v, [&](int i) { return -a.d[i]; });
-}
-ND_DUAL bool operator<(Duals<S, N> a, Duals<S, N> b) { return a.v < b.v; }
-ND_DUAL bool operator>(Duals<S, N> a, Duals<S, N> b) { return a.v > b.v; }
-ND_DUAL bool operator<=(Duals<S, N> a, Duals<S, N> b) { return a.v <= b.v; }
-ND_DUAL bool operator>=(Duals<S, N> a, Duals<S, N> b) { return a.v >= b.v; }
-ND_DUAL bool operator==(Duals<S, N> a, Duals<S, N> b) { return a.v == b.v; }
-ND_DUAL bool operator!=(Duals<S, N> a, Duals<S, N> b) { return a.v != b.v; }
-
-// A function of one argument with value f and derivative g there.
-ND_DUAL1 chain(S f, S g, const Duals<S, N>& a) {
-  return mkds<N>(f, [&](int i) { return g * a.d[i]; });
-}
-ND_DUAL1 sin(Duals<S, N> a) { return chain(sin(a.v), cos(a.v), a); }
-ND_DUAL1 cos(Duals<S, N> a) { return chain(cos(a.v), -sin(a.v), a); }
-ND_DUAL1 tan(Duals<S, N> a) {
-  const S t = tan(a.v);
-  return chain(t, S(1) + t * t, a);
-}
-ND_DUAL1 asin(Duals<S, N> a) {
-  const Divisor<S> by(sqrt(max(S(1) - a.v * a.v, S(1e-30))));
-  return mkds<N>(asin(a.v), [&](int i) { return by(a.d[i]); });
-}
-ND_DUAL1 acos(Duals<S, N> a) {
-  const Divisor<S> by(sqrt(max(S(1) - a.v * a.v, S(1e-30))));
-  return mkds<N>(acos(a.v), [&](int i) { return by(-a.d[i]); });
-}
-ND_DUAL1 atan(Duals<S, N> a) {
-  const Divisor<S> by(S(1) + a.v * a.v);
-  return mkds<N>(atan(a.v), [&](int i) { return by(a.d[i]); });
-}
-ND_DUAL1 atan2(Duals<S, N> y, Duals<S, N> x) {
-  const S r2 = x.v * x.v + y.v * y.v;
-  const Divisor<S> by(r2);
-  return mkds<N>(atan2(y.v, x.v), [&](int i) { return r2 > S(0) ? by(x.v * y.d[i] - y.v * x.d[i]) : S(0); });
-}
-ND_DUAL1 sinh(Duals<S, N> a) { return chain(sinh(a.v), cosh(a.v), a); }
-ND_DUAL1 cosh(Duals<S, N> a) { return chain(cosh(a.v), sinh(a.v), a); }
-ND_DUAL1 tanh(Duals<S, N> a) {
-  const S t = tanh(a.v);
-  return chain(t, S(1) - t * t, a);
-}
-ND_DUAL1 exp(Duals<S, N> a) {
-  const S e = exp(a.v);
-  return chain(e, e, a);
-}
-ND_DUAL1 exp2(Duals<S, N> a) {
-  const S e = exp2(a.v);
-  return chain(e, e * S(0.6931471805599453), a);
-}
-ND_DUAL1 log(Duals<S, N> a) {
-  const Divisor<S> by(a.v);
-  return mkds<N>(log(a.v), [&](int i) { return by(a.d[i]); });
-}
-ND_DUAL1 log2(Duals<S, N> a) {
-  const Divisor<S> by(a.v * S(0.6931471805599453));
-  return mkds<N>(log2(a.v), [&](int i) { return by(a.d[i]); });
-}
-ND_DUAL1 sqrt(Duals<S, N> a) {
-  const S s = sqrt(a.v);
-  const Divisor<S> by(S(2) * s);
-  return mkds<N>(s, [&](int i) { return s > S(0) ? by(a.d[i]) : S(0); });
-}
-ND_DUAL1 inverseSqrt(Duals<S, N> a) {
-  const S r = S(1) / sqrt(a.v);
-  return chain(r, S(-0.5) * r * r * r, a);
-}
-ND_DUAL1 pow(Duals<S, N> x, Duals<S, N> y) {
-  if (x.v < S(0)) return Duals<S, N>(S(0) / S(0), 0);
-  const S p = pow(x.v, y.v);
-  // y x^(y - 1): FP64 duals take the power from p, in place of a second 64-bit power
-  const S g = y.v * (std::is_same<S, double>::value && x.v > S(0) && p > S(0) ? p / x.v : pow(x.v, y.v - S(1)));
-  return mkds<N>(p, [&](int i) {
-    S dp = S(0);
-    if (x.d[i] != S(0)) dp += g * x.d[i];
-    if (y.d[i] != S(0) && x.v > S(0)) dp += p * log(x.v) * y.d[i];
-    return dp;
-  });
-}
-ND_DUAL1 floor(Duals<S, N> a) { return Duals<S, N>(floor(a.v), 0); }
-ND_DUAL1 ceil(Duals<S, N> a) { return Duals<S, N>(ceil(a.v), 0); }
-ND_DUAL1 trunc(Duals<S, N> a) { return Duals<S, N>(trunc(a.v), 0); }
-ND_DUAL1 round(Duals<S, N> a) { return Duals<S, N>(round(a.v), 0); }
-ND_DUAL1 abs(Duals<S, N> a) { return a.v < S(0) ? -a : a; }
-ND_DUAL1 sign(Duals<S, N> a) {
-  return Duals<S, N>(a.v > S(0) ? S(1) : (a.v < S(0) ? S(-1) : S(0)), 0);
-}
-ND_DUAL1 min(Duals<S, N> a, Duals<S, N> b) { return b.v < a.v ? b : a; }
-ND_DUAL1 max(Duals<S, N> a, Duals<S, N> b) { return b.v > a.v ? b : a; }
-ND_DUAL1 fma(Duals<S, N> a, Duals<S, N> b, Duals<S, N> c) { return a * b + c; }
-ND_DUAL1 radians(Duals<S, N> a) { return chain(a.v * S(0.017453292519943295), S(0.017453292519943295), a); }
-ND_DUAL1 degrees(Duals<S, N> a) { return chain(a.v * S(57.29577951308232), S(57.29577951308232), a); }
-ND_DUAL1 select(Duals<S, N> f, Duals<S, N> t, bool c) { return c ? t : f; }
-ND_DUAL void sin_cos(Duals<S, N> x, Duals<S, N>& s, Duals<S, N>& c) {
-  const S sv = sin(x.v), cv = cos(x.v);
-  s = chain(sv, cv, x);
-  c = chain(cv, -sv, x);
-}
-#undef ND_DUAL1
-#undef ND_DUAL
-
 }  // namespace ndw

@@ -1558,7 +1558,8 @@ class FormulaCompiler:
         angle = self.mul_angle(s)
         if angle is not None:
             cname = cpp_name(s.name)
-            self.declare(s.name, TE(MUL_ANGLE, cname, None, lvalue=False), s.line)
+            inv = self.inv_fn and self.is_inv(s.init)
+            self.declare(s.name, TE(MUL_ANGLE, cname, None, lvalue=False, inv=inv), s.line)
             return f"const ndw::MulAngle<T> {cname} = {angle};"
         if s.init is not None:
             te = self.expr(s.init)

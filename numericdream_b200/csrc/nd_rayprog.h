@@ -48,6 +48,7 @@ ND_DEV_INLINE float load_ro(const float* p) { return __ldg(p); }
 ND_DEV_INLINE int32_t float_bits(float x) { return __float_as_int(x); }
 ND_DEV_INLINE int32_t floor_int(float x) { return __float2int_rd(x); }  // saturates; NaN -> 0
 ND_DEV_INLINE uint32_t low_word(double x) { return uint32_t(__double2loint(x)); }
+ND_DEV_INLINE double double_below(double x) { return __longlong_as_double(__double_as_longlong(x) - 1); }  // of x > 0
 ND_DEV_INLINE uint16_t half_bits(float x) { return __half_as_ushort(__float2half_rn(x)); }
 #else
 // host builds of this header are compiled with -ffp-contract=off
@@ -72,6 +73,13 @@ ND_DEV_INLINE uint32_t low_word(double x) {
   uint64_t b;
   memcpy(&b, &x, sizeof(b));
   return uint32_t(b);
+}
+ND_DEV_INLINE double double_below(double x) {
+  uint64_t b;
+  memcpy(&b, &x, sizeof(b));
+  --b;
+  memcpy(&x, &b, sizeof(b));
+  return x;
 }
 // IEEE binary16 bits of x, rounded to nearest even (host builds of the ray program)
 ND_DEV_INLINE uint16_t half_bits(float x) {
@@ -168,13 +176,16 @@ ND_DEV_INLINE double div_known(double a, double b, double y) {
   return fma_d(fma_d(-q1, b, a), y, q1);
 }
 
-// 1 / sqrt(s) with both operations correctly rounded, from y, an approximation of it to
-// about an ulp: the same corrections, first for the root, then for its reciprocal (whose
-// one exception, a divisor of all ones, divides).
+// 1 / sqrt(s) with both operations correctly rounded, from y, an approximation of it to a
+// few ulps: the same corrections, first for the root, then for its reciprocal (whose one
+// exception is a divisor of all ones).  The corrected root is an ulp off when the exact one
+// lies within 2^-53 or so of an ulp of a midpoint; g is the rounded root just when s is
+// within g ulps(g) of g^2 (Tuckerman's test), and what does not pass divides and takes the
+// root instead (so does the upper half of a power of two's neighbourhood, whose ulp changes).
 ND_DEV_INLINE double inv_sqrt_from(double s, double y) {
   const double g0 = rn_mul(s, y);
   const double g = fma_d(fma_d(-g0, g0, s), 0.5 * y, g0);
-  if (low_word(g) == 0xffffffffu) return 1.0 / g;
+  if (low_word(g) == 0xffffffffu || !(fabs(fma_d(-g, g, s)) < rn_mul(g, g - double_below(g)))) return 1.0 / sqrt(s);
   const double y1 = fma_d(fma_d(-g, y, 1.0), y, y);
   return fma_d(fma_d(-g, y1, 1.0), y1, y1);
 }

@@ -64,7 +64,8 @@ ND_HD_INLINE float nd_atan2_max(float ax, float ay) {
   asm("max.NaN.ftz.f32 %0, %1, %2;\n\tmax.NaN.ftz.f32 %0, %0, %3;" : "=&f"(m) : "f"(ax), "f"(ay), "f"(1.17549435e-38f));
   return m;
 #else
-  return ax != ax || ay != ay ? ax + ay : fmaxf(fmaxf(ax, ay), 1.17549435e-38f);
+  const float m = ax != ax || ay != ay ? ax + ay : fmaxf(ax, ay);
+  return m == 0.0f ? 1.17549435e-38f : m;  // a subnormal stays: the host does not flush it
 #endif
 }
 // mx == mn ? 1 : q, as a selection: left to itself the compiler branches around the

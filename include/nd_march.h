@@ -227,7 +227,9 @@ typedef struct nd_gbuffer {
   float* shade;       /* Lambert grey level (simple_geometry, template.wgsl:4492) */
   float* shadow;      /* shadow-ray visibility in [0, 1] (1 without a shadow ray) */
   double* depth64;    /* t in FP64 */
-  uint32_t* evals;    /* DE evaluations spent on this ray */
+  uint32_t* evals;    /* DE evaluations the algorithm asks for on this ray (a bisection sample at
+                         an FP32 position whose distance is already known counts like any other,
+                         although its evaluation is saved: with ND_VIEW_EXACT_HIT, many do) */
   uint16_t* normal_half; /* the normal as the reference's RGBA16F target: 4 IEEE halves per ray,
                             w = 1 on a hit (8-byte aligned) */
 } nd_gbuffer;
@@ -253,8 +255,9 @@ typedef struct nd_march_opts {
 
 typedef struct nd_stats {
   uint64_t rays;
-  uint64_t de_evals;        /* all DE evaluations: march, normals, shadows and trap pass */
-  uint64_t march_evals;     /* primary march probes + refinement */
+  uint64_t de_evals;        /* all DE evaluations, counted as nd_gbuffer.evals: march, normals, shadows
+                               and trap pass */
+  uint64_t march_evals;     /* primary march probes + refinement, whichever kernel ran them */
   uint64_t normal_evals;
   uint64_t shadow_evals;
   uint64_t trap_evals;      /* one DE with the orbit trap per hit (when trap/iters are requested) */

@@ -434,13 +434,13 @@ def profile_forward(args):
     g = runtime.GBuffer.allocate(workloads.rays(views))
     opts = runtime.make_opts(kernel=abi.ND_KERNEL_PERSISTENT, refill_threshold=4)
     ctx.forward(views, g, opts)
-    march_ms = []
+    kernel_ms = []
     if args.repeat > 0:
         flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
         for _ in range(args.repeat):
             flush.fill_(1)
             ctx.forward(views, g, opts)
-            march_ms.append(ctx.stats().march_ms)
+            kernel_ms.append((ctx.stats().march_ms, ctx.stats().shade_ms))
     if args.with_lite:
         lite = abi.make_lite([((0.05, 0.05, 0.22), 0.0, 0.2, 1.3), ((1.0, 0.95, 0.82), 1.0, 0.8, 1.7)],
                              [(abi.ND_LIGHT_GLOBAL, (0.4, 0.8, -0.45), (1.0, 0.95, 0.9), 1.2)])
@@ -449,13 +449,22 @@ def profile_forward(args):
     st = ctx.stats()
     line = {"workload": args.workload, "views": len(views), "rays": workloads.rays(views), "de_evals": st.de_evals,
             "march_evals": st.march_evals, "normal_evals": st.normal_evals, "hits": st.hits}
-    if march_ms:
-        m = sorted(march_ms)[len(march_ms) // 2]
-        line.update({"march_ms_median": m, "sm_ns_per_march_eval": m * 1e6 * torch.cuda.get_device_properties(0).multi_processor_count
-                                              / max(st.march_evals, 1)})
+    if kernel_ms:
+        march, shade = (sorted(k)[len(kernel_ms) // 2] for k in zip(*kernel_ms))
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        # (over both kernels: the surface pass takes the bisections of an FP32 march)
+        line.update({"march_ms_median": march, "shade_ms_median": shade,
+                     "sm_ns_per_eval": (march + shade) * 1e6 * sms / max(st.de_evals, 1)})
     print(json.dumps(line))
     ctx.close()
     return 0
+
+
+def forward_tflops(st, flops_per_eval, march_ms, shade_ms):
+    """TFLOP/s of a forward's DE evaluations over the device time of its march and its surface
+    pass.  An FP32 march leaves its bisections to the surface pass, so that neither kernel's
+    time goes with march_evals alone."""
+    return st.de_evals * flops_per_eval / ((march_ms + shade_ms) * 1e-3) / 1e12
 
 
 def small_and_deepzoom(ctx, sptr, timed, steps, with_errors=True):
@@ -774,10 +783,9 @@ def main():
         from numericdream_b200 import opcount
 
         flops_per_eval, per = opcount.flops_per_eval_for(views)
-        flops = st.march_evals * flops_per_eval  # the march kernel's evaluations
         nominal = opcount.fp32_peak_tflops(clk.get("sm_mhz") or clk.get("sm_max_mhz"))
         peak = measured_fp32 if measured_fp32 else nominal
-        achieved = flops / (kms[0] * 1e-3) / 1e12
+        achieved = forward_tflops(st, flops_per_eval, *kms)
         cpu, err = None, None
         if not args.no_cpu:
             c = run_cpu(views, seconds_budget=10.0, with_fp64=True)
@@ -822,8 +830,9 @@ def main():
                          "issue_note": "the march's share of issue slots busy (ncu smsp__issue_active, one "
                                        "capture): the bound of this scalar, branchy code, whose FP32 "
                                        "add/mul/fma are under half of the instructions it issues",
-                         "kernel": "persistent_kernel (march); FLOPs = its DE evaluations x FLOPs per "
-                                   "evaluation, over its CUDA-event time",
+                         "kernel": "persistent_kernel (march) and shade_kernel (surface pass); FLOPs = the "
+                                   "forward's DE evaluations x FLOPs per evaluation, over the CUDA-event time of "
+                                   "both (the surface pass takes the march's bisections)",
                          "kernel_ms": kms[0], "shade_pass_ms": kms[1],
                          "flops_per_eval": flops_per_eval, "sfu_per_eval": per["sfu"],
                          "peak_source": ("measured: nd_measure_fp32_peak, independent FFMA chains on this GPU "

@@ -367,12 +367,10 @@ ND_DEV_INLINE DEOut<T> formula_de_p(ndw::v3<T> pos, const PR& p, const nd_trap_d
       // fixed point: every later update would see this same carry (the one just
       // recorded), so nothing changes any more
       if (!ch && !(c.dr != drp)) break;
-#if !defined(ND_OPCOUNT_BUILD)  // the op count is of the reference's loop, which runs every iteration
     } else if constexpr (F::kSettles) {
       bool settled = false;
       c = F::template step<T, PR>(c, pos, p, settled);
       if (settled) break;
-#endif
     } else {
       c = F::template step<T, PR>(c, pos, p);
     }

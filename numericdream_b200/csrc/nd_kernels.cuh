@@ -293,7 +293,13 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
   const bool queue = a.shadow_queue != nullptr;
   const int64_t count = list ? int64_t(*a.hit_count) : a.total_rays;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  uint32_t taps = 0, shadow = 0, bisect = 0, lost = 0;
+  uint32_t taps = 0, shadow = 0, bisect = 0, lost = 0, late = 0;
+  // the watchdog of a bisection with a budget of hundreds of samples, which the march left
+  // here (the start is in shared memory: an FP64 DE leaves no registers for it)
+  __shared__ int64_t started;
+  if (threadIdx.x == 0) started = globaltimer_ns();
+  __syncthreads();
+  const auto expired = [&]() { return globaltimer_ns() > started + a.deadline_ns; };
   for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); i0 < count; i0 += stride) {
     const int64_t i = i0 + lane;  // the loop bound is warp-uniform: every lane takes part in the ballot
     bool want = false;
@@ -315,10 +321,13 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
         bool hit = true;
         if (list) {
           int used = 0;
-          hit = resolve_hit<Set, T, kDir64, kScenes>(v, dir, h, a.scenes, &t, &used);
+          const Resolved how = resolve_hit<Set, T, kDir64, kScenes>(v, dir, h, a.scenes, expired, &t, &used);
+          hit = how == RESOLVED_HIT;
           bisect += uint32_t(used);
           h.evals += uint32_t(used);
-          if (!hit) {
+          if (how == RESOLVED_LATE) {
+            ++late;
+          } else if (!hit) {
             ++lost;
             write_miss(v, a.out, r, h.evals);
           }
@@ -365,6 +374,7 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
       shadow += __shfl_xor_sync(full, shadow, o);
       bisect += __shfl_xor_sync(full, bisect, o);
       lost += __shfl_xor_sync(full, lost, o);
+      late += __shfl_xor_sync(full, late, o);
     }
     if (lane == 0 && taps + shadow + bisect) {
       atomicAdd(&a.stats->normal_evals, (unsigned long long)taps);
@@ -372,7 +382,11 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
       atomicAdd(&a.stats->march_evals, (unsigned long long)bisect);
       atomicAdd(&a.stats->de_evals, (unsigned long long)taps + shadow + bisect);
     }
-    if (lane == 0 && lost) atomicAdd(&a.stats->hits, 0ull - lost);
+    if (lane == 0 && lost + late) atomicAdd(&a.stats->hits, 0ull - lost - late);
+    if (lane == 0 && late) {  // neither finished nor written
+      atomicAdd(&a.stats->rays, 0ull - late);
+      atomicAdd(&a.stats->timeouts, 1u);
+    }
   }
 }
 

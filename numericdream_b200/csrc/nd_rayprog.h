@@ -1310,20 +1310,22 @@ namespace nd {
 
 // The hit of a listed ray: the bisection between the last sample above eps and the first
 // below it, as Lane::advance runs it inline.  *t: the hit distance, *used: the samples it
-// took.  False when march_to's loop runs out of samples first (max_steps 0): a miss.
+// took.  RESOLVED_MISS when march_to's loop runs out of samples first (max_steps 0),
+// RESOLVED_LATE when `expired`, asked every 64 samples, ends a long bisection.
 //
 // A bisection that runs its whole budget (exact_hit) soon halves a bracket that spans
 // one or two FP32 positions: a sample at a position whose DE one of the bracket's ends
 // has is taken from there (it counts as a sample like any other).
-template <class Set, class T, bool kDir64, bool kScenes = false>
-ND_DEV_INLINE bool resolve_hit(const DevView& v, const Dir<kDir64>& dir, const HitEntry& h, const DevScene* scenes,
-                               double* t, int* used) {
+enum Resolved { RESOLVED_HIT, RESOLVED_MISS, RESOLVED_LATE };
+template <class Set, class T, bool kDir64, bool kScenes, class Expired>
+ND_DEV_INLINE Resolved resolve_hit(const DevView& v, const Dir<kDir64>& dir, const HitEntry& h, const DevScene* scenes,
+                                   const Expired& expired, double* t, int* used) {
   double a = h.a, b = h.b;
   *used = 0;
   *t = b;
-  if (v.verify != 0 || !(v.refine > 0 && (v.exact_hit ? b > a : b - a > march_eps<T>(v, b)))) return true;
+  if (v.verify != 0 || !(v.refine > 0 && (v.exact_hit ? b > a : b - a > march_eps<T>(v, b)))) return RESOLVED_HIT;
   int n = h.steps + 1;
-  if (n >= v.max_samples) return false;
+  if (n >= v.max_samples) return RESOLVED_MISS;
   const D3 o = d3(v.org[0], v.org[1], v.org[2]), d = dir.get();
   ndw::v3<T> pa = to_t<T>(fmadd(o, d, a)), pb = to_t<T>(fmadd(o, d, b));
   T da = T(0), db = T(0);
@@ -1349,10 +1351,11 @@ ND_DEV_INLINE bool resolve_hit(const DevView& v, const Dir<kDir64>& dir, const H
       known_a = true;
     }
     if ((b - a <= march_eps<T>(v, st) && !v.exact_hit) || *used >= v.refine) break;
-    if (n >= v.max_samples) return false;
+    if (n >= v.max_samples) return RESOLVED_MISS;
+    if ((*used & 63) == 0 && expired()) return RESOLVED_LATE;
   }
   *t = b;
-  return true;
+  return RESOLVED_HIT;
 }
 
 // The orbit trap and changed-iteration count at a ray's hit point: the formula

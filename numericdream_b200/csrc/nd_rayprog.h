@@ -180,20 +180,33 @@ ND_DEV_INLINE double div_known(double a, double b, double y) {
 // few ulps: the same corrections, first for the root, then for its reciprocal (whose one
 // exception is a divisor of all ones).  The corrected root is an ulp off when the exact one
 // lies within 2^-53 or so of an ulp of a midpoint; g is the rounded root just when s is
-// within g ulps(g) of g^2 (Tuckerman's test), and what does not pass divides and takes the
-// root instead (so does the upper half of a power of two's neighbourhood, whose ulp changes).
-ND_DEV_INLINE double inv_sqrt_from(double s, double y) {
+// within g ulps(g) of g^2 (Tuckerman's test).  False when either does not hold (and in the
+// upper half of a power of two's neighbourhood, whose ulp changes): the caller divides.
+ND_DEV_INLINE bool inv_sqrt_steps(double s, double y, double* inv) {
   const double g0 = rn_mul(s, y);
   const double g = fma_d(fma_d(-g0, g0, s), 0.5 * y, g0);
-  if (low_word(g) == 0xffffffffu || !(fabs(fma_d(-g, g, s)) < rn_mul(g, g - double_below(g)))) return 1.0 / sqrt(s);
   const double y1 = fma_d(fma_d(-g, y, 1.0), y, y);
-  return fma_d(fma_d(-g, y1, 1.0), y1, y1);
+  *inv = fma_d(fma_d(-g, y1, 1.0), y1, y1);
+  return low_word(g) != 0xffffffffu && fabs(fma_d(-g, g, s)) < rn_mul(g, g - double_below(g));
 }
+ND_DEV_INLINE double inv_sqrt_from(double s, double y) {
+  double inv;
+  return inv_sqrt_steps(s, y, &inv) ? inv : 1.0 / sqrt(s);
+}
+// The direction of a ray takes this; the division and the root, which hardly ever run, stay
+// out of line (inlined beside the steps they cost the plain launch spilled registers: 256 x
+// 256 rays 308 -> 331 us).  The headlight's one root a hit divides: 308 us against 315.
+#if defined(__CUDA_ARCH__)
+static __device__ __noinline__ double inv_sqrt_divided(double s) { return 1.0 / sqrt(s); }
+#endif
 ND_DEV_INLINE double inv_sqrt(double s) {
 #if defined(__CUDA_ARCH__)
-  if (s > 1e-200 && s < 1e200) return inv_sqrt_from(s, ::rsqrt(s));
-#endif
+  double inv;
+  if (inv_sqrt_steps(s, ::rsqrt(s), &inv) && s > 1e-200 && s < 1e200) return inv;
+  return inv_sqrt_divided(s);
+#else
   return 1.0 / sqrt(s);
+#endif
 }
 
 struct Stats {
@@ -819,7 +832,7 @@ ND_DEV_INLINE float lambert(const DevView& v, D3 dir, double nx, double ny, doub
     kx = rn_add(rn_add(-dir.x, rn_mul(v.uup[0], 0.45)), -rn_mul(v.uright[0], 0.35));
     ky = rn_add(rn_add(-dir.y, rn_mul(v.uup[1], 0.45)), -rn_mul(v.uright[1], 0.35));
     kz = rn_add(rn_add(-dir.z, rn_mul(v.uup[2], 0.45)), -rn_mul(v.uright[2], 0.35));
-    const double inv = inv_sqrt(rn_add(rn_add(rn_mul(kx, kx), rn_mul(ky, ky)), rn_mul(kz, kz)));
+    const double inv = 1.0 / sqrt(rn_add(rn_add(rn_mul(kx, kx), rn_mul(ky, ky)), rn_mul(kz, kz)));
     kx *= inv; ky *= inv; kz *= inv;
   }
   // explicitly rounded (no FMA contraction), so that every kernel gives the same bits

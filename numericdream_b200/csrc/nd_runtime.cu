@@ -557,10 +557,14 @@ nd_status enqueue(nd_ctx* ctx, const nd_view_desc* views, int nviews, const nd_m
       const bool accel = plan_voxels[p] > 0;
       // Untuned, one view with no more rays than the persistent grid has lanes runs the
       // plain launch: with one ray per lane there is nothing to refill, and the plain
-      // loop has no ballot per pass and no second pass for the normals (10 % faster on
-      // a 256 x 256 Mandelbulb).
+      // loop has no ballot per pass and no second pass for the normals.  The grid is taken as
+      // 9 blocks of 128 an SM, the most that a march of few registers holds, where this
+      // formula's holds 7 or 8 (plain and persistent, 12-iteration Mandelbulb: 256 x 256 rays
+      // 136 and 147 us, 440 x 340 172 and 202, 500 x 330 167 and 191; Mandelbox: 74 and 82,
+      // 127 and 151, 125 and 154).  With an FP64 DE, where it is 0.82 to 1.14 of the persistent
+      // march's time by formula and shadows, it is the march's own residency.
       if (!(opts && opts->kernel) && !tu.tuned && nv == 1 && !accel && sc.nscenes == 0 && L.table.resident_b128 &&
-          rays <= int64_t(L.table.resident_b128(0)) * ctx->num_sms * 128)
+          rays <= int64_t(std::max(prec == 64 ? 0 : 9, L.table.resident_b128(0))) * ctx->num_sms * 128)
         kernel = ND_KERNEL_PLAIN;
       if (accel && kernel == ND_KERNEL_PLAIN) {
         if (opts && opts->kernel == ND_KERNEL_PLAIN)

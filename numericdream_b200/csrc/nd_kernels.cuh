@@ -81,9 +81,11 @@ __global__ void __launch_bounds__(128, MinBlocks<T>::value) plain_kernel(const _
   const int64_t thread = lane < a.chunk ? warp * a.chunk + lane : v.rays;
   // The ray index inside the view.  A warp of a 8 x 4 pixel block has more of its lanes
   // alike than one of 32 pixels in a row: an FP32 view of 256 x 256 takes 281 us against
-  // 291.  With fewer warps than would keep the schedulers busy nothing is gained (96 x 54
-  // rays: 186 against 184 us), nor with an FP64 DE; the persistent march, whose lanes
-  // drift apart as they refill, was 1 to 3 % slower with it.
+  // 291.  Rows and blocks, Mandelbulb and Mandelbox: 120 x 75 rays 102 and 106, 99 and 102
+  // us; 128 x 128 120 and 116, 71 and 71; 160 x 110 112 and 114, 75 and 72; 192 x 128 124
+  // and 116, 92 and 91; 440 x 340 174 and 177, 126 and 127.  So with fewer warps than would
+  // keep the schedulers busy nothing is gained, nor with an FP64 DE; the persistent march,
+  // whose lanes drift apart as they refill, was 1 to 3 % slower with it.
   const bool blocks = sizeof(T) == 4 && v.rays >= 16384 && thread < v.rays;
   const int64_t local = blocks ? block_order(v, thread) : thread;
   unsigned long long rays = 0, hits = 0, m = 0, nn = 0, sh = 0;

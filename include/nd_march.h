@@ -389,7 +389,8 @@ nd_status nd_graph_capture_scenes(nd_ctx* ctx, const nd_view_desc* views, int32_
  * (silhouette) changes are not differentiated.  opts (nullable) selects the dual
  * numbers' precision, de_precision 32 (default) or 64; its other fields are unused.
  * Needs a directional light (light_dir), central-difference normals and no shadow
- * ray; other views return ND_ERR_UNSUPPORTED.  Synchronises the stream. */
+ * ray; other views return ND_ERR_UNSUPPORTED.  Synchronises the stream.  The context keeps
+ * lists of 44 bytes per ray, of at most 2^22 rays (185 MB), until it is destroyed. */
 nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, const nd_orbit_camera* cams, int32_t nviews,
                             const int32_t* param_idx, int32_t nparams, const nd_gbuffer* fwd,
                             const float* dL_dshade, double* dL_dtheta, double* dshade_dtheta,
@@ -401,7 +402,7 @@ nd_status nd_march_backward(nd_ctx* ctx, const nd_view_desc* views, const nd_orb
  * allocation may synchronise the device, loops that must not allocate after
  * start-up).  Runs the persistent kernel on the current device and the given
  * stream; its scratch (view table, work counters, statistics) is a fixed array of
- * about 28 KB inside the library, present on every GPU that loads it.
+ * about 45 KB inside the library, present on every GPU that loads it.
  * Limits: at most 64 views and 2^31-1 rays per call; trap and iters outputs are
  * not available here (they need per-ray scratch) and return ND_ERR_UNSUPPORTED.
  * The call cannot be captured into a CUDA graph (it copies the view table from its

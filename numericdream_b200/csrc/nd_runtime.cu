@@ -1817,7 +1817,7 @@ size_t nd_sizeof(const char* name) {
 // because it may synchronise the device, and embedded or real-time loops that must
 // not allocate after start-up.  nd_march_forward_noalloc serves them with the
 // persistent kernel and no context: its only scratch (the view table, the work
-// counters and the statistics block, about 28 KB) lives in the file-scope array
+// counters and the statistics block, about 45 KB) lives in the file-scope array
 // below, which the library's module brings with it on every GPU that loads the
 // library, until the process exits.
 namespace {

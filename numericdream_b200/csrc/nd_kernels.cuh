@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::value * 128 / kBlock)
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  typename std::conditional<kDefer, MarchLane<T, kDir64>, Lane<T, kDir64>>::type L;
+  typename std::conditional<kDefer, MarchLane<T, kDir64, (Set::kCount > 1)>, Lane<T, kDir64>>::type L;
   L.item = -1;
   L.view = 0;
   L.hit = false;
@@ -303,9 +303,12 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
   uint32_t taps = 0, shadow = 0, bisect = 0, lost = 0, late = 0;
   // the watchdog of a bisection with a budget of hundreds of samples, which the march left
   // here (the start is in shared memory: an FP64 DE leaves no registers for it)
+  constexpr bool kBisects = Set::kCount == 1;
   __shared__ int64_t started;
-  if (threadIdx.x == 0) started = globaltimer_ns();
-  __syncthreads();
+  if constexpr (kBisects) {
+    if (threadIdx.x == 0) started = globaltimer_ns();
+    __syncthreads();
+  }
   const auto expired = [&]() { return globaltimer_ns() > started + a.deadline_ns; };
   for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); i0 < count; i0 += stride) {
     const int64_t i = i0 + lane;  // the loop bound is warp-uniform: every lane takes part in the ballot
@@ -326,17 +329,19 @@ __global__ void __launch_bounds__(128, ShadeBlocks<T>::value)
         Dir<kDir64> dir;
         dir.set(ray_dir(v, local));
         bool hit = true;
-        if (list) {
-          int used = 0;
-          const Resolved how = resolve_hit<Set, T, kDir64, kScenes>(v, dir, h, a.scenes, expired, &t, &used);
-          hit = how == RESOLVED_HIT;
-          bisect += uint32_t(used);
-          h.evals += uint32_t(used);
-          if (how == RESOLVED_LATE) {
-            ++late;
-          } else if (!hit) {
-            ++lost;
-            write_miss(v, a.out, r, h.evals);
+        if constexpr (kBisects) {
+          if (list) {
+            int used = 0;
+            const Resolved how = resolve_hit<Set, T, kDir64, kScenes>(v, dir, h, a.scenes, expired, &t, &used);
+            hit = how == RESOLVED_HIT;
+            bisect += uint32_t(used);
+            h.evals += uint32_t(used);
+            if (how == RESOLVED_LATE) {
+              ++late;
+            } else if (!hit) {
+              ++lost;
+              write_miss(v, a.out, r, h.evals);
+            }
           }
         }
         if (list && hit) {

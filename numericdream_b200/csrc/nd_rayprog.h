@@ -411,6 +411,7 @@ ND_DEV_INLINE DEOut<T> formula_de(ndw::v3<T> pos, const float* params, const nd_
 // gives NO_SURFACE_DE (1e6) / the carry unchanged.
 template <class... Fs> struct FormulaSet;
 template <class F> struct FormulaSet<F> {
+  static constexpr int kCount = 1;
   template <class T, bool kTrap = false>
   static ND_DEV_INLINE DEOut<T> de(int, ndw::v3<T> pos, const DevView& v) {
     return formula_de<F, T, kTrap>(pos, v.params, v.trap, v.factor, &v.image);
@@ -443,6 +444,7 @@ template <class F> struct FormulaSet<F> {
   }
 };
 template <class F, class G, class... Rest> struct FormulaSet<F, G, Rest...> {
+  static constexpr int kCount = 2 + int(sizeof...(Rest));
   template <class T, bool kTrap = false>
   static ND_DEV_INLINE DEOut<T> de(int code, ndw::v3<T> pos, const DevView& v) {
     if (code == 0) return formula_de<F, T, kTrap>(pos, v.params, v.trap, v.factor, &v.image);
@@ -1160,12 +1162,18 @@ template <class T, bool kDir64> struct Lane {
 //   pass 2898 + 521 us with the bisection in the march, 2508 + 651 without; FP64, two views
 //   of 40 exact bisections 3719 + 146 and 2590 + 1044, a close-up that stops at eps 5231 +
 //   719 and 5123 + 1354;
+//   a formula group's (kGroup) bisections stay in the march.  Its surface pass, with one
+//   call site more for the group's DE, is compiled with other fused products: normals of the
+//   four-formula batch's Mandelbulbs moved by 4e-4 (2-norm), and the hits of a few rays.  Nor
+//   was it faster: that batch, march and surface pass, 4.98 + 1.39 ms with the bisection
+//   there, 5.31 + 0.93 without; with 40 exact FP32 bisections 5.01 + 3.49 and 8.46 + 0.89, a
+//   share of it with 40 exact FP64 ones 3.95 + 6.00 and 5.85 + 1.09.
 //   i counts the probes and k the samples after them (the one below eps, the bisection's),
 //   so a view that bisects has taken i + k samples, and while probing the limit on the
 //   samples is not below the one on the steps; n counts a verified march's samples.
-template <class T, bool kDir64> struct MarchLane {
+template <class T, bool kDir64, bool kGroup> struct MarchLane {
   enum : int32_t { kProbe, kBisect, kVerify, kRefine, kDone };
-  static constexpr bool kBisects = sizeof(T) == 8;
+  static constexpr bool kBisects = sizeof(T) == 8 || kGroup;
   int32_t item;  // work-item index inside the launch, -1 when idle
   int32_t view;
   int32_t mode;
@@ -1252,17 +1260,18 @@ template <class T, bool kDir64> struct MarchLane {
   }
 
   // One sample of a bisection, or the sample below eps that starts it.  False: the ray is
-  // at its hit, with the bracket [a, st] as far as it goes.
+  // at its hit, or at the bracket [a, st] of one that the surface pass bisects.
   ND_DEV_INLINE bool bisect(const DevView& v, bool below) {
     if (mode == kProbe) {
-      if (v.exact_hit || !(v.refine > 0 && st - a > march_eps<T>(v, st))) return false;
+      if (!kGroup && v.exact_hit) return false;
+      if (!(v.refine > 0 && (v.exact_hit ? st > a : st - a > march_eps<T>(v, st)))) return false;
       b = st;
       mode = kBisect;
     } else {
       const double e = march_eps<T>(v, st);
       if (below) b = st;
       else a = st;
-      if (b - a <= e || k >= v.refine) {
+      if ((b - a <= e && !v.exact_hit) || k >= v.refine) {
         ++k;
         a = st = b;
         return false;

@@ -452,7 +452,7 @@ def profile_forward(args):
     if kernel_ms:
         march, shade = (sorted(k)[len(kernel_ms) // 2] for k in zip(*kernel_ms))
         sms = torch.cuda.get_device_properties(0).multi_processor_count
-        # (over both kernels: the surface pass takes the bisections of an FP32 march)
+        # (over both kernels: an FP32 march of one formula leaves its bisections to the surface pass)
         line.update({"march_ms_median": march, "shade_ms_median": shade,
                      "sm_ns_per_eval": (march + shade) * 1e6 * sms / max(st.de_evals, 1)})
     print(json.dumps(line))
@@ -462,8 +462,8 @@ def profile_forward(args):
 
 def forward_tflops(st, flops_per_eval, march_ms, shade_ms):
     """TFLOP/s of a forward's DE evaluations over the device time of its march and its surface
-    pass.  An FP32 march leaves its bisections to the surface pass, so that neither kernel's
-    time goes with march_evals alone."""
+    pass.  An FP32 march of one formula leaves its bisections to the surface pass, so that
+    neither kernel's time goes with march_evals alone."""
     return st.de_evals * flops_per_eval / ((march_ms + shade_ms) * 1e-3) / 1e12
 
 
@@ -832,7 +832,7 @@ def main():
                                        "add/mul/fma are under half of the instructions it issues",
                          "kernel": "persistent_kernel (march) and shade_kernel (surface pass); FLOPs = the "
                                    "forward's DE evaluations x FLOPs per evaluation, over the CUDA-event time of "
-                                   "both (the surface pass takes the march's bisections)",
+                                   "both (a march of one formula leaves its bisections to the surface pass)",
                          "kernel_ms": kms[0], "shade_pass_ms": kms[1],
                          "flops_per_eval": flops_per_eval, "sfu_per_eval": per["sfu"],
                          "peak_source": ("measured: nd_measure_fp32_peak, independent FFMA chains on this GPU "

@@ -267,7 +267,8 @@ typedef struct nd_stats {
   uint32_t kernel;          /* kernel that ran (ND_KERNEL_PLAIN / _PERSISTENT) */
   double march_ms;          /* device time of the march kernels of the last nd_march_forward
                                (CUDA events on its stream; 0 after a graph launch) */
-  double shade_ms;          /* device time of its shade passes (hit bisection, normals, shadows, orbit trap) */
+  double shade_ms;          /* device time of its shade passes (hit bisection of a single formula's
+                               march, normals, shadows, orbit trap) */
   uint64_t accel_voxels;    /* accelerator grid cells built (one DE evaluation each, not in de_evals) */
   double accel_ms;          /* device time of the accelerator grid builds */
 } nd_stats;
